@@ -2459,29 +2459,31 @@ int launch_factor(const Symbolic& sy, T* L, T* U, const double* vals, const int6
       }
       if (ps.syrk_big.ctas > 0) {
         if constexpr (std::is_same<T, double>::value) {
-          if (oz && ps.ozaki) {
-            // digits of the panel rows, then the update on the integer tensor pipe
-            launch_ozaki_slice(L, fr.l_off, fr.m, fr.k, tasks + ps.oz_slice.off, prefix + ps.oz_slice.pre,
-                               aux + ps.oz_slice.off, ps.oz_slice.count, ps.oz_slice.ctas, ps.j0, *oz, s);
-            cudaEvent_t ev[2] = {nullptr, nullptr};
-            if (oz_ev) {
-              while (oz_ev->size() < 2 * (*oz_used + 1)) {
-                cudaEvent_t e;
-                if (cudaEventCreate(&e) != cudaSuccess) break;
-                oz_ev->push_back(e);
+          if (oz && !ps.ozaki.empty()) {
+            // residues of a group's panel rows, then its update on the integer tensor pipe
+            for (const OzGroup& g : ps.ozaki) {
+              launch_ozaki_residues(L, fr.l_off, fr.m, fr.k, tasks + g.residues.off, prefix + g.residues.pre,
+                                    aux + g.residues.off, g.residues.count, g.residues.ctas, ps.j0, *oz, s);
+              cudaEvent_t ev[2] = {nullptr, nullptr};
+              if (oz_ev) {
+                while (oz_ev->size() < 2 * (*oz_used + 1)) {
+                  cudaEvent_t e;
+                  if (cudaEventCreate(&e) != cudaSuccess) break;
+                  oz_ev->push_back(e);
+                }
+                if (oz_ev->size() >= 2 * (*oz_used + 1)) {
+                  ev[0] = (*oz_ev)[2 * *oz_used];
+                  ev[1] = (*oz_ev)[2 * *oz_used + 1];
+                  ++*oz_used;
+                  cudaEventRecord(ev[0], s);
+                }
               }
-              if (oz_ev->size() >= 2 * (*oz_used + 1)) {
-                ev[0] = (*oz_ev)[2 * *oz_used];
-                ev[1] = (*oz_ev)[2 * *oz_used + 1];
-                ++*oz_used;
-                cudaEventRecord(ev[0], s);
-              }
+              launch_ozaki_update(L, U, fr.l_off, fr.u_off, fr.m, fr.k, tasks + g.tiles.off, prefix + g.tiles.pre,
+                                  aux + g.tiles.off, g.tiles.count, g.tiles.ctas, ps.j0, *oz, err, s);
+              if (ev[1]) cudaEventRecord(ev[1], s);
+              launches += 2;
             }
-            launch_ozaki_update(L, U, fr.l_off, fr.u_off, fr.m, fr.k, tasks + ps.syrk_big.off,
-                                prefix + ps.syrk_big.pre, aux + ps.syrk_big.off, ps.syrk_big.count,
-                                ps.syrk_big.ctas, ps.j0, *oz, err, s);
-            if (ev[1]) cudaEventRecord(ev[1], s);
-            ++launches;
+            --launches;
           } else {
             k_syrk_big_dmma<<<grid_of(2 * ps.syrk_big.ctas), kBigThreads, dmma_smem(), s>>>(
                 L, U, fr, tasks + ps.syrk_big.off, prefix + ps.syrk_big.pre, ps.syrk_big.count, ps.j0);
@@ -2773,7 +2775,7 @@ int64_t GpuCholesky::bytes_needed(const Symbolic& sy, int nrhs_max, int precisio
   int64_t b = fel * sy.u_elems + el * (sy.wvec_elems * nr + sy.solve_partials * nr + sy.solve_slots * kPanel * nr);
   b += std::max(1, std::min(nslots, kMaxSlots)) * slot_bytes(sy, precision_bytes);
   if (fel != el) b += slot_bytes(sy, (int)fel);  // the FP64 work factor of a demoted setup
-  if (fel == 8) b += sy.oz_rows_max * ((int64_t)kOzSlices * kOzK + 4);  // digit slices + exponents
+  if (fel == 8) b += sy.oz_rows_max * ((int64_t)kOzModuli * kOzK + 4);  // residues + exponents
   b += 8 * (int64_t)sy.task_aux.size();
   b += 8 * (int64_t)(sy.l_off.size() + sy.u_off.size() + sy.wvec_off.size() + sy.entry_dst.size() +
                      sy.rel_off.size() + sy.rows_off.size() + sy.task_prefix.size() + sy.dinv_off.size());
@@ -2825,7 +2827,7 @@ std::string GpuCholesky::setup(Symbolic&& sy, const std::vector<int>& perm_to_ve
   if (!(e = upload(&d_task_aux_, sy_.task_aux, s)).empty()) return e;
   if (fac_elem_ == 8 && ozaki_ && sy_.oz_rows_max > 0) {
     oz_.rows = sy_.oz_rows_max;
-    if (!(e = alloc((void**)&oz_.slices, (size_t)kOzSlices * kOzK * oz_.rows)).empty()) return e;
+    if (!(e = alloc((void**)&oz_.residues, (size_t)kOzModuli * kOzK * oz_.rows)).empty()) return e;
     if (!(e = alloc((void**)&oz_.exps, sizeof(int) * (size_t)oz_.rows)).empty()) return e;
     if (!(e = ozaki_setup(oz_)).empty()) return e;
   }

@@ -90,10 +90,10 @@ class GpuCholesky {
   void set_tensor_core_update(bool on) { tc_update_ = on; }
   // FP64 factorization: the trailing updates the analysis planned for it (large
   // outer panels, kOzRowsCap rows per launch at most) run on the integer tensor
-  // pipe by digit splitting (ozaki_update.h) instead of the FP64 tensor pipe.  On
+  // pipe by residues (ozaki_update.h) instead of the FP64 tensor pipe.  On
   // by default; takes effect at setup().
   void set_ozaki(bool on) { ozaki_ = on; }
-  bool ozaki() const { return oz_.slices != nullptr; }
+  bool ozaki() const { return oz_.residues != nullptr; }
   // Records CUDA events around every integer-pipe update launch of the following
   // factorizations; take_ozaki_ms() returns their summed device time (after the
   // stream has completed them) and starts over.

@@ -684,7 +684,7 @@ std::string analyse(int n, const int64_t* rowptr, const int* colind, const doubl
     }
     int kmax = 0;
     for (int s : lp.fronts) kmax = std::max(kmax, sy.front_k[s]);
-    // TDEM_OZAKI_ALL=1 plans every trailing update that fits the digit buffer on the
+    // TDEM_OZAKI_ALL=1 plans every trailing update that fits the residue buffer on the
     // integer tensor pipe (tests of small models)
     const char* oz_all = std::getenv("TDEM_OZAKI_ALL");
     const double oz_min_flops = (oz_all && oz_all[0] == '1') ? 0.0 : kOzMinFlops;
@@ -733,35 +733,40 @@ std::string analyse(int n, const int64_t* rowptr, const int* colind, const doubl
       add_tasks(sy, ps.syrk_rest, frest, c6b);
       add_tasks(sy, ps.syrk_big, fbig, c5);
       {
-        // the Ozaki path: slice-buffer rows of the fronts, in task order
-        int64_t rows = 0;
+        // the Ozaki path: groups of fronts whose panel rows fit the residue buffer
         double fl = 0.0;
-        std::vector<int64_t> c7;
-        for (size_t q = 0; q < fbig.size(); ++q) {
-          const int s = fbig[q], k = sy.front_k[s], m = sy.front_m[s];
-          const int J1 = std::min(k, J0 + kOuter);
-          sy.task_aux[ps.syrk_big.off + q] = rows;
-          rows += m - J1;
-          fl += (double)(m - J1) * (m - J1) * (J1 - J0);
-          c7.push_back(cdiv(m - J1, 64));
+        int64_t most = 0;
+        for (int s : fbig) {
+          const int64_t J1 = std::min(sy.front_k[s], J0 + kOuter), r = sy.front_m[s] - J1;
+          fl += (double)r * r * (J1 - J0);
+          most = std::max(most, r);
         }
-        if (!fbig.empty() && rows <= kOzRowsCap && fl >= oz_min_flops) {
-          ps.ozaki = true;
-          ps.oz_rows = rows;
-          // 128 x 64 output tiles (the right half of a last 128-column tile past the
-          // front is skipped) x K blocks of 64 digits x the kept digit pairs
-          for (int s : fbig) {
-            const int k = sy.front_k[s], m = sy.front_m[s];
-            const int J1 = std::min(k, J0 + kOuter);
-            const int64_t r = m - J1, nt = cdiv(r, 128);
-            const int64_t ctas = nt * (nt + 1) - ((r - (nt - 1) * 128) <= 64 ? 1 : 0);
-            const int64_t kpad = cdiv(J1 - J0, 64) * 64;
-            sy.oz_macs += (double)ctas * 128.0 * 64.0 * (double)kpad * (kOzSlices * (kOzSlices + 1) / 2);
-          }
-          sy.oz_rows_max = std::max(sy.oz_rows_max, rows);
+        if (!fbig.empty() && most <= kOzRowsCap && fl >= oz_min_flops) {
           sy.oz_flops += fl;
-          add_tasks(sy, ps.oz_slice, fbig, c7);
-          for (size_t q = 0; q < fbig.size(); ++q) sy.task_aux[ps.oz_slice.off + q] = sy.task_aux[ps.syrk_big.off + q];
+          for (size_t q = 0; q < fbig.size();) {
+            std::vector<int> grp;
+            std::vector<int64_t> first, c7, c8;
+            int64_t rows = 0;
+            for (; q < fbig.size(); ++q) {
+              const int s = fbig[q];
+              const int64_t J1 = std::min(sy.front_k[s], J0 + kOuter), r = sy.front_m[s] - J1;
+              if (rows + r > kOzRowsCap) break;
+              grp.push_back(s);
+              first.push_back(rows);
+              c7.push_back(cdiv(r, 64));
+              c8.push_back(oz_tiles(r));
+              // 256 x 96 output tiles x K padded to 128 x the moduli
+              sy.oz_macs += (double)c8.back() * 256.0 * kOzTileCols * (double)(cdiv(J1 - J0, 128) * 128) * kOzModuli;
+              rows += r;
+            }
+            OzGroup g;
+            add_tasks(sy, g.residues, grp, c7);
+            add_tasks(sy, g.tiles, grp, c8);
+            for (size_t i = 0; i < grp.size(); ++i)
+              sy.task_aux[g.residues.off + i] = sy.task_aux[g.tiles.off + i] = first[i];
+            ps.ozaki.push_back(g);
+            sy.oz_rows_max = std::max(sy.oz_rows_max, rows);
+          }
         }
       }
       add_tasks(sy, ps.solve_upd, fr, c4);

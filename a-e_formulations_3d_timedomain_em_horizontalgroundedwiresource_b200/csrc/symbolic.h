@@ -30,14 +30,27 @@ constexpr int kSolveRows = 256;  // rows per CTA of the solve updates
 constexpr int kSolveChunk = 8;   // 64 x 64 blocks accumulated by one level-solve unit
 constexpr int kUnitInts = 16;    // ints per level-solve unit record (64 bytes)
 constexpr int kSolveLookahead = 8;  // extra blocks a chain unit takes ahead of its newest one
-// Trailing updates on the integer tensor pipe (FP64 by the Ozaki splitting): each
-// row of the outer panel is split into kOzSlices signed 7-bit digits after scaling
-// by a power of two; only launches whose panels total at most kOzRowsCap rows (the
-// slice buffer) and at least kOzMinFlops flops take that path.
-constexpr int kOzSlices = 8;
-constexpr int kOzK = kOuter;          // digits per row and slice (K of an outer panel, padded)
-constexpr int64_t kOzRowsCap = 1 << 19;
+// Trailing updates on the integer tensor pipe (FP64 by the Ozaki scheme II): each row
+// of the outer panel is scaled by a power of two, rounded to integers and reduced
+// modulo kOzModuli moduli; the steps of at least kOzMinFlops flops take that path, in
+// launches whose panels total at most kOzRowsCap rows (the residue buffer: 1.07 GB).
+constexpr int kOzModuli = 16;
+constexpr int kOzK = kOuter;          // residues per row and modulus (K of an outer panel, padded)
+constexpr int64_t kOzRowsCap = 1 << 17;
 constexpr double kOzMinFlops = 2e9;
+// Tiles of an update of r rows: 256 rows (a CTA pair) x 96 columns, in super-columns of
+// eight column tiles (768 columns, three row tiles); inside one the row tiles from its
+// diagonal down, where the first reaches three of the columns and the second six.
+constexpr int kOzTileCols = 96, kOzSuper = 8;
+inline int64_t oz_tiles(int64_t r) {
+  const int64_t rows = (r + 255) / 256, cols = (r + kOzTileCols - 1) / kOzTileCols;
+  int64_t n = 0;
+  for (int64_t c = 0, below = rows; c < cols; c += kOzSuper, below -= 3) {
+    const int64_t w = cols - c < kOzSuper ? cols - c : kOzSuper;
+    n += (w < 3 ? w : 3) + (below > 1 ? (w < 6 ? w : 6) : 0) + (below > 2 ? (below - 2) * w : 0);
+  }
+  return n;
+}
 // most blocks one level-solve unit accumulates (a chain unit, or a short row)
 constexpr int kUnitBlocks = (kSolveLookahead + 1 > kSolveChunk + 1) ? kSolveLookahead + 1 : kSolveChunk + 1;
 
@@ -59,6 +72,14 @@ struct TaskList {
   int64_t ctas = 0;    // total CTAs
 };
 
+// Fronts whose trailing update shares one launch on the integer tensor pipe: the panel
+// rows [J1, m) are reduced front after front (task_aux of both lists' entries: the
+// front's first row in the residue buffer) by `residues` (64 rows per CTA), then
+// `tiles` (oz_tiles of each) multiplies them.
+struct OzGroup {
+  TaskList residues, tiles;
+};
+
 // One 64-wide inner panel [j0, j1) of the factorization, j1 = min(k, j0 + 64).  The
 // outer panel is [J0, J1), J0 = floor(j0 / kOuter) * kOuter, J1 = min(k, J0 + kOuter).
 struct PanelStep {
@@ -71,12 +92,9 @@ struct PanelStep {
   // [j1, j1 + 64) (syrk_next) and the tiles right of it (syrk_rest)
   TaskList syrk_next, syrk_rest;
   TaskList syrk_big;   // at the end of an outer panel: trailing [J1, m) by [J0, J1), 128-tiles
-  // Ozaki path of syrk_big (ozaki true): the panel rows [J1, m) of every front of
-  // syrk_big are split into digits, front after front (task_aux of the syrk_big
-  // entries: the front's first row in the slice buffer), by oz_slice (64 rows per CTA)
-  bool ozaki = false;
-  int64_t oz_rows = 0;
-  TaskList oz_slice;
+  // Ozaki path of syrk_big (not empty): the fronts of syrk_big in groups that fit the
+  // residue buffer, one after another
+  std::vector<OzGroup> ozaki;
   TaskList solve_upd;  // ceil((m - j1) / kSolveRows) CTAs per front (fwd update / bwd partials)
 };
 
@@ -140,7 +158,7 @@ struct Symbolic {
   double flops = 0.0;         // factorization flops
   double oz_flops = 0.0;      // flops of the trailing updates on the Ozaki path
   double oz_macs = 0.0;       // 8-bit multiply-adds those updates issue on the tensor pipe
-  int64_t oz_rows_max = 0;    // slice-buffer rows the Ozaki path needs
+  int64_t oz_rows_max = 0;    // residue-buffer rows the Ozaki path needs
   int max_m = 0, max_k = 0;
   int64_t solve_partials = 0; // scratch entries per RHS column for backward partial sums
 };

@@ -241,8 +241,8 @@ typedef struct tdem_plan_info {
   uint64_t digest;          /* hash of the elimination order, the fronts, the entry map and the
                                solve units: equal digests mean identical launch plans */
   double ozaki_flops;       /* flops of the trailing updates planned on the integer tensor
-                               pipe (FP64 products by digit splitting; FP64 solvers) */
-  int64_t ozaki_rows;       /* rows of the digit buffer those updates need */
+                               pipe (FP64 products by residues; FP64 solvers) */
+  int64_t ozaki_rows;       /* rows of the residue buffer those updates need */
   int64_t solve_chain;      /* 64-wide pivot blocks on the critical path of one triangular
                                solve direction: the sum over the tree levels of the largest
                                front's pivot blocks (each is one dependent link) */
