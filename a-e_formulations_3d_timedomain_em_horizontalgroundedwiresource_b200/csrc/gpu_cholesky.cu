@@ -55,6 +55,8 @@ __device__ __forceinline__ T* felem(T* L, T* U, int64_t lo, int64_t uo, int m, i
 
 __device__ __forceinline__ double tsqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float tsqrt(float x) { return sqrtf(x); }
+__device__ __forceinline__ double trsqrt(double x) { return rsqrt(x); }
+__device__ __forceinline__ float trsqrt(float x) { return 1.0f / sqrtf(x); }
 
 // ---------------------------------------------------------------------------
 // factorization kernels
@@ -104,116 +106,224 @@ __global__ void k_extend_add(T* __restrict__ L, T* __restrict__ U, Fronts f, con
   for (int a = b + lane; a < rc; a += 32) *felem(L, U, lo, uo, mp, kp, rl[a], pc) += uc[a + (int64_t)b * rc];
 }
 
-// Cholesky of the w x w diagonal block of panel [j0, j0 + w) (one CTA of 256
-// threads per front), right-looking in shared memory with one barrier per column.
-// Thread t owns row i = t % 64 and, of it, the columns c = t / 64 (mod 4).  Step j
-// scales column j on the fly (L(r, j) = A(r, j) / sqrt(A(j, j)), recomputed by
-// every thread that needs it) and subtracts L(i, j) L(c, j) from A(i, c) for
-// j < c <= i; the finished column goes to the upper triangle A[j][r] (r > j) and
-// the diagonal to diag[j], which no later step reads, so column j is read
-// unchanged throughout its step.  Same operations in the same order per element
-// as a column-at-a-time factorization: the result does not depend on the thread
-// layout.
-// With dinv (FP64 factorization) the CTA also inverts the finished block into the
-// front's inverted diagonal blocks (dinv_off[s] + 64 * 64 * (j0 / 64), column-major,
-// leading dimension w): the operand of the panel solve k_trsm_dmma and of the
-// triangular solves (by 16 x 16 blocks, see below).
+__device__ __forceinline__ void dmma16816(double (&c)[4], const double (&a)[8], const double (&b)[4]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, "
+      "{%12,%13,%14,%15}, {%0,%1,%2,%3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]),
+        "d"(b[1]), "d"(b[2]), "d"(b[3]));
+}
+
+// c += a b for one warp: a(16 x K), b(K x 8), K = 8 or 16, as functions of (row, column);
+// lane (g, q) = (lane / 4, lane % 4) holds c(g + 8 (i / 2), 2 q + i % 2) in c[i].
+template <int K, class FA, class FB>
+__device__ __forceinline__ void mul16x8(double (&c)[4], FA&& a, FB&& b, int g, int q) {
+  double af[K / 2], bf[K / 4];
+#pragma unroll
+  for (int i = 0; i < K / 2; ++i) af[i] = a(g + 8 * (i & 1), q + 4 * (i >> 1));
+#pragma unroll
+  for (int i = 0; i < K / 4; ++i) bf[i] = b(q + 4 * i, g);
+  if constexpr (K == 16)
+    dmma16816(c, af, bf);
+  else
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(af[0]), "d"(af[1]), "d"(af[2]), "d"(af[3]), "d"(bf[0]), "d"(bf[1]));
+}
+template <int K, class FA, class FB>
+__device__ __forceinline__ void mul16x8(float (&c)[4], FA&& a, FB&& b, int g, int q) {
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] = fmaf(a(g + 8 * (i >> 1), k), b(k, 2 * q + (i & 1)), c[i]);
+}
+
+// Cholesky of the w x w diagonal block of panel [j0, j0 + w) (one CTA of 256 threads
+// per front) in shared memory, eight columns at a time: each of 64 threads (one per row)
+// factors the 8 x 8 diagonal block M D M^T in its own registers, solves its row against
+// it, and all warps update what is right of it with the FP64 tensor pipe.  With dinv
+// (FP64 factorization) the CTA also inverts the finished block into the front's
+// inverted diagonal blocks (dinv_off[s] + 64 * 64 * (j0 / 64), column-major, leading
+// dimension w): the operand of the panel solve k_trsm_dmma and of the triangular solves.
+// The inverse goes by 16-wide block rows, X_ij = -X_ii sum_{j <= k < i} L_ik X_kj, made
+// by the six other warps while the next columns are factored.
+//
+// The bound is the chain of 64 pivots at the FP64 pipe's latency (25 cycles an
+// instruction, 50 a reciprocal): a reciprocal, a product and a multiply-add each, about
+// 100 cycles, with nothing between threads inside the eight columns.  With a block-wide
+// barrier, a square root, a division and shared-memory round trips per column the kernel
+// took 67 us for one front; a 16 x 16 diagonal block in one warp by shuffles 300 cycles a
+// column and 20 us; this takes 15 us.
 template <class T>
 __global__ void __launch_bounds__(256) k_potrf(T* __restrict__ L, Fronts f, const int* __restrict__ fronts, int j0,
                                                int* __restrict__ err, const int* __restrict__ c0_of,
                                                T* __restrict__ dinv = nullptr,
                                                const int64_t* __restrict__ dinv_off = nullptr) {
-  __shared__ T A[P][P + 1];
-  __shared__ T diag[P];
+  constexpr int QB = 16, CB = 8, LD = P + 2;
+  // A(r, c), r >= c: the block, then its factor L(r, c).  A(c, r), r > c: the inverse
+  // X(r, c) from its block row on; its diagonal is xd (the reciprocals of the factor's).
+  // Rows of 528 bytes: a thread's own row and the diagonal block go by 16-byte accesses.
+  // (CB rows more than the block: the last 16-row tile of an update may reach past it.)
+  __shared__ __align__(16) T A[P + CB][LD];
   __shared__ T xd[P];
-  __shared__ T tb[3][16][16];  // band products of the blocked inverse
+  __shared__ T tb[3][QB][QB + 1];  // sums of the inverse's block row
   const int s = fronts[blockIdx.x];
   const int m = f.m[s], k = f.k[s];
   const int w = min(P, k - j0);
+  const int nb = (w + QB - 1) / QB, wp = nb * QB;
   T* F = L + f.l_off[s];
-  for (int idx = threadIdx.x; idx < w * w; idx += blockDim.x) {
-    const int i = idx % w, j = idx / w;
-    A[i][j] = (i >= j) ? F[(j0 + i) + (int64_t)(j0 + j) * m] : (T)0;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int tr = t & (P - 1), tc = t >> 6;  // this thread's row, and columns tc + 4 q, of the copies
+  {
+    T v[P / 4];
+#pragma unroll
+    for (int q = 0; q < P / 4; ++q) {
+      const int j = tc + 4 * q;  // padded to whole blocks with the identity
+      v[q] = (tr == j) ? (T)1 : (T)0;
+      if (tr < w && j <= tr) v[q] = F[(j0 + tr) + (int64_t)(j0 + j) * m];
+    }
+#pragma unroll
+    for (int q = 0; q < P / 4; ++q) A[tr][tc + 4 * q] = v[q];
+    for (int q = t; q < CB * LD; q += 256) A[P + q / LD][q % LD] = (T)0;
   }
+  auto Xv = [&](int r, int c) -> T {
+    const T v = A[c][r], e = xd[c];
+    return r == c ? e : (r > c ? v : (T)0);
+  };
+  // the inverse's block row kb: this warp's column block and half
+  const int xj = (warp - 2) >> 1, xh = (warp & 1) * 8, g = lane >> 2, q4 = lane & 3;
+  auto inverse_sum = [&](int kb) {  // sum_{xj <= l < kb} L(kb, l) X(l, xj)
+    T u[4] = {(T)0, (T)0, (T)0, (T)0};
+    for (int l = xj; l < kb; ++l)
+      mul16x8<QB>(u, [&](int r, int c) { return A[kb * QB + r][l * QB + c]; },
+                  [&](int r, int c) { return Xv(l * QB + r, xj * QB + xh + c); }, g, q4);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) tb[xj][g + 8 * (i >> 1)][xh + 2 * q4 + (i & 1)] = u[i];
+  };
+  auto inverse_row = [&](int kb) {  // X(kb, xj) = -X(kb, kb) times the sum
+    T u[4] = {(T)0, (T)0, (T)0, (T)0};
+    mul16x8<QB>(u, [&](int r, int c) { return Xv(kb * QB + r, kb * QB + c); },
+                [&](int r, int c) { return tb[xj][r][xh + c]; }, g, q4);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) A[xj * QB + xh + 2 * q4 + (i & 1)][kb * QB + g + 8 * (i >> 1)] = -u[i];
+  };
+  auto inverse_diag = [&](int kb, int c) {  // column c of X(kb, kb): L y = e_c
+    const int o = kb * QB;
+    T y[QB];
+#pragma unroll
+    for (int r = 0; r < QB; ++r) y[r] = (r == c) ? (T)1 : (T)0;
+#pragma unroll
+    for (int j = 0; j < QB; ++j) {
+      y[j] *= xd[o + j];
+#pragma unroll
+      for (int r = j + 1; r < QB; ++r) y[r] = fma(-A[o + r][o + j], y[j], y[r]);
+      if (j > c) A[o + c][o + j] = y[j];
+    }
+  };
   __syncthreads();
-  const int i = threadIdx.x & (P - 1), g = threadIdx.x >> 6;
-  for (int j = 0; j < w; ++j) {
-    T d = A[j][j];
-    if (!(d > (T)0)) {
-      if (threadIdx.x == 0) atomicCAS(err, 0, c0_of[s] + j0 + j + 1);
-      d = (T)1;
+  for (int o = 0; o < wp; o += CB) {
+    if (t < P) {
+      T M[CB][CB], x[CB], dj[CB];
+#pragma unroll
+      for (int i = 0; i < CB; ++i)
+#pragma unroll
+        for (int c = 0; c <= i; ++c) M[i][c] = A[o + i][o + c];
+      T* row = &A[t][o];
+#pragma unroll
+      for (int c = 0; c < CB; ++c) x[c] = row[c];
+      asm volatile("bar.sync 1, 64;" ::: "memory");  // both warps hold the block before its rows change
+#pragma unroll
+      for (int j = 0; j < CB; ++j) {
+        const T d = M[j][j] > (T)0 ? M[j][j] : (T)1;
+        dj[j] = d;
+        const T rc = (T)1 / d;
+        T u[CB];
+#pragma unroll
+        for (int i = j + 1; i < CB; ++i) u[i] = M[i][j] * rc;
+#pragma unroll
+        for (int i = j + 1; i < CB; ++i)
+#pragma unroll
+          for (int c = j + 1; c <= i; ++c) M[i][c] = fma(-u[i], M[c][j], M[i][c]);
+#pragma unroll
+        for (int i = j + 1; i < CB; ++i) M[i][j] = u[i];
+      }
+      // the row times L^-T = M^-T D^-1/2 (a row of the block itself: its row of L)
+#pragma unroll
+      for (int c = 0; c < CB; ++c)
+#pragma unroll
+        for (int e = c + 1; e < CB; ++e) x[e] = fma(-x[c], M[e][c], x[e]);
+      T mine = (T)1;
+#pragma unroll
+      for (int c = 0; c < CB; ++c) {
+        mine = t == o + c ? dj[c] : mine;
+        const T inv = trsqrt(dj[c]);
+        x[c] *= inv;
+        if (t == o) xd[o + c] = inv;
+      }
+      const T root = tsqrt(mine);
+      if (t >= o && t < wp) {
+#pragma unroll
+        for (int c = 0; c < CB; ++c) row[c] = t == o + c ? root : x[c];
+      }
+      if (t == o) {
+        int bad = CB;
+#pragma unroll
+        for (int j = CB - 1; j >= 0; --j) bad = M[j][j] > (T)0 ? bad : j;
+        if (bad < CB) atomicCAS(err, 0, c0_of[s] + j0 + o + bad + 1);
+      }
+    } else if (dinv != nullptr && o >= QB) {
+      // meanwhile the inverse's previous block row: sums and diagonal block, then products
+      const int kb = o / QB - 1;
+      if (o % QB == 0) {
+        if (xj < kb) inverse_sum(kb);
+        if (warp == 7 && lane < QB) inverse_diag(kb, lane);
+      } else if (xj < kb) {
+        inverse_row(kb);
+      }
     }
-    const T sd = tsqrt(d);
-    const T inv = (T)1 / sd;
-    if (i > j && i < w) {
-      const T lij = A[i][j] * inv;
-      // first column of this thread's group after j
-      int c = j + 1 + ((g - (j + 1)) & 3);
-      for (; c <= i; c += 4) A[i][c] -= lij * (A[c][j] * inv);
-      if (g == 0) A[j][i] = lij;
+    __syncthreads();
+    // rank-8 update of the lower triangle right of the columns, 16 x 8 tiles
+    const int n = (wp - o - CB + QB - 1) / QB, tiles = n * (n + 1);
+#pragma unroll
+    for (int it = 0; it < 3; ++it) {
+      const int tile = warp + 8 * it;
+      if (tile >= tiles) break;
+      const int bi = tile < 2 ? 0 : (tile < 6 ? 1 : (tile < 12 ? 2 : 3)), h = tile - bi * (bi + 1);
+      const int r0 = o + CB + QB * bi, c0 = o + CB + 8 * h;
+      T u[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) u[i] = A[r0 + g + 8 * (i >> 1)][c0 + 2 * q4 + (i & 1)];
+      mul16x8<CB>(u, [&](int r, int c) { return -A[r0 + r][o + c]; }, [&](int r, int c) { return A[c0 + c][o + r]; },
+                  g, q4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + g + 8 * (i >> 1), c = c0 + 2 * q4 + (i & 1);
+        if (r >= c && r < wp) A[r][c] = u[i];
+      }
     }
-    if (threadIdx.x == 0) diag[j] = sd;
     __syncthreads();
   }
-  for (int idx = threadIdx.x; idx < w * w; idx += blockDim.x) {
-    const int r = idx % w, c = idx / w;
-    if (r >= c) F[(j0 + r) + (int64_t)(j0 + c) * m] = (r == c) ? diag[c] : A[c][r];
+#pragma unroll
+  for (int q = 0; q < P / 4; ++q) {
+    const int j = tc + 4 * q;
+    if (tr < w && j <= tr) F[(j0 + tr) + (int64_t)(j0 + j) * m] = A[tr][j];
   }
   if (dinv == nullptr) return;
-  // L(r, c) = A[c][r] (r > c) or diag[r]; the inverse X(r, c) (r > c) goes to the
-  // lower triangle, whose working values are dead, and its diagonal to xd.  By
-  // 16 x 16 blocks: the diagonal blocks by substitution, four threads per column
-  // running X(r, c) = -(sum_{c <= l < r} L(r, l) X(l, c)) / L(r, r) over at most 15
-  // rows; then the blocks below them band by band, X_ij = -X_ii sum_{j <= k < i}
-  // L_ik X_kj, every element of a band at once (a column-long substitution would
-  // chain 63 dependent steps).
-  constexpr int QB = 16;
-  auto Xv = [&](int l, int c) -> T { return l == c ? xd[c] : (l > c ? A[l][c] : (T)0); };
-  {
-    const int c = threadIdx.x >> 2, part = threadIdx.x & 3;
-    const unsigned mask = 0xFu << ((threadIdx.x & 31) & ~3);
-    if (c < w) {
-      const int bend = min(w, (c / QB + 1) * QB);
-      if (part == 0) xd[c] = (T)1 / diag[c];
-      __syncwarp(mask);
-      for (int r = c + 1; r < bend; ++r) {
-        T sum = (T)0;
-        for (int l = c + part; l < r; l += 4) sum = fma(A[l][r], l == c ? xd[c] : A[l][c], sum);
-        sum += __shfl_xor_sync(mask, sum, 1);
-        sum += __shfl_xor_sync(mask, sum, 2);
-        if (part == 0) A[r][c] = -sum / diag[r];
-        __syncwarp(mask);
-      }
-    }
+  if (warp >= 2) {
+    if (xj < nb - 1) inverse_sum(nb - 1);
+  } else if (t < QB) {
+    inverse_diag(nb - 1, t);
   }
   __syncthreads();
-  const int nb = (w + QB - 1) / QB;
-  for (int d = 1; d < nb; ++d) {
-    const int np = nb - d;  // block pairs (j + d, j) of band d
-    for (int e = threadIdx.x; e < np * QB * QB; e += blockDim.x) {
-      const int j = e / (QB * QB), rr = (e / QB) % QB, cc = e % QB;
-      const int r = (j + d) * QB + rr, c = j * QB + cc;
-      T t = (T)0;
-      if (r < w && c < w)
-        for (int l = j * QB; l < (j + d) * QB; ++l) t = fma(A[l][r], Xv(l, c), t);
-      tb[j][rr][cc] = t;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < np * QB * QB; e += blockDim.x) {
-      const int j = e / (QB * QB), rr = (e / QB) % QB, cc = e % QB;
-      const int i0 = (j + d) * QB, r = i0 + rr, c = j * QB + cc;
-      if (r < w && c < w) {
-        T x = (T)0;
-        for (int l = i0; l <= r; ++l) x = fma(Xv(r, l), tb[j][l - i0][cc], x);
-        A[r][c] = -x;
-      }
-    }
-    __syncthreads();
-  }
+  if (warp >= 2 && xj < nb - 1) inverse_row(nb - 1);
+  __syncthreads();
   T* D = dinv + dinv_off[s] + (int64_t)(j0 / P) * P * P;
-  for (int q = threadIdx.x; q < w * w; q += blockDim.x) {
-    const int r = q % w, c = q / w;
-    D[q] = (r > c) ? A[r][c] : (r == c ? xd[c] : (T)0);
+#pragma unroll
+  for (int q = 0; q < P / 4; ++q) {
+    const int j = tc + 4 * q;
+    if (tr < w && j < w) D[tr + j * w] = Xv(tr, j);
   }
 }
 
@@ -460,15 +570,6 @@ constexpr int kLdC = kTileBig + 2;   // 130, epilogue tile columns (fits in the 
 constexpr int KD = 16;               // K per stage of the tensor-pipe update (one k16 step)
 constexpr int kDStages = 4;          // stage buffers (three chunks in flight)
 static_assert(kBigCols * kLdC <= kDStages * KD * (kLdA + kLdB), "epilogue tile must fit the operand buffers");
-
-__device__ __forceinline__ void dmma16816(double (&c)[4], const double (&a)[8], const double (&b)[4]) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, "
-      "{%12,%13,%14,%15}, {%0,%1,%2,%3};"
-      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]),
-        "d"(b[1]), "d"(b[2]), "d"(b[3]));
-}
 
 // Panel triangular solve on the FP64 tensor pipe: rows [j1, m) of the panel columns
 // times L_dd^-T, with L_dd^-1 the inverse k_potrf wrote (dinv_off[s] + 64 * 64 *
