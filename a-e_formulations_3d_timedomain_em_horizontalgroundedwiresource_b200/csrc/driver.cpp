@@ -664,8 +664,9 @@ std::string TransientSolve::step(int itime, int t1, int t2, double m1, double m2
     return "time grid needs a restart layer older than the history ring holds";
   const double* u1 = layer(t1);
   const double* u2 = (t2 >= 0) ? layer(t2) : layer(t1);
+  // the layer this step fills is the scratch (none of the layers it reads, see above)
   launch_history_rhs(d_rowptr_, d_col_, d_C_, u1, u2, m1, (t2 >= 0) ? m2 : 0.0, d_S_, coef, d_bound_, n_, npls_,
-                     d_rhs_, s_);
+                     d_rhs_, layer(itime), s_);
   if (ps_) {
     const std::string se = anomaly_source(itime, t1, t2);
     if (!se.empty()) return se;
@@ -1074,12 +1075,13 @@ std::string TransientSolve::time_step(bool block, int reps, double* ms) {
   const double* u = layer(0);  // any finite history: only the time is measured
   auto one = [&]() -> std::string {
     if (block) {
-      launch_history_rhs(d_rowptr_, d_col_, d_C_, u, u, 1.0, 0.0, d_S_, 0.0, d_bound_, n_, npls_, d_rhs_, s_);
+      launch_history_rhs(d_rowptr_, d_col_, d_C_, u, u, 1.0, 0.0, d_S_, 0.0, d_bound_, n_, npls_, d_rhs_, layer(1),
+                         s_);
       return chol_->solve_graph(d_rhs_, d_x_, n_, npls_, s_, slot_);
     }
     for (int j = 0; j < npls_; ++j) {
       launch_history_rhs(d_rowptr_, d_col_, d_C_, u + j * n, u + j * n, 1.0, 0.0, d_S_ + j * n, 0.0, d_bound_, n_,
-                         1, d_rhs_ + j * n, s_);
+                         1, d_rhs_ + j * n, nullptr, s_);
       chol_->solve(d_rhs_ + j * n, d_x_ + j * n, n_, 1, s_, slot_);
     }
     return "";

@@ -160,65 +160,77 @@ __global__ void k_history_rhs(const int64_t* __restrict__ rowptr, const int* __r
   }
 }
 
-// Several sources: one warp per row, the sources in groups of 8.  Lane l takes the
-// entries q = b + l, b + l + 32, ... of the row (the row's columns and values are
-// read once per group, not once per source) and sums its products for the 8
-// sources; the 32 lanes' sums are combined by recursive halving (each round a
-// lane keeps half of its values and adds its partner's other half), after which
-// lane l holds the row total of source 4 ((l >> 4) & 1) + 2 ((l >> 3) & 1) +
-// ((l >> 2) & 1) of the group.  The additions happen in an order fixed by the
-// lane pattern alone.
-__global__ void k_history_rhs_multi(const int64_t* __restrict__ rowptr, const int* __restrict__ col,
-                                    const double* __restrict__ C, const double* __restrict__ u1,
-                                    const double* __restrict__ u2, double m1c, double m2c,
-                                    const double* __restrict__ S, double coef, const uint8_t* __restrict__ bound,
-                                    int n, int npls, double* __restrict__ rhs) {
-  const int row = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= n) return;
-  if (bound[row]) {
-    for (int p = lane; p < npls; p += 32) rhs[row + (int64_t)p * n] = 0.0;
-    return;
+// Several sources: v[j][p] = m1 u1(j, p) + m2 u2(j, p), source-contiguous, so that a
+// row's entry reads the values of all its sources side by side (32 edges x 32 sources a
+// CTA, turned through shared memory).
+__global__ void __launch_bounds__(256) k_history_combine(const double* __restrict__ u1, const double* __restrict__ u2,
+                                                         double m1c, double m2c, int n, int npls,
+                                                         double* __restrict__ v) {
+  __shared__ double tile[32][33];
+  const int j0 = blockIdx.x * 32, p0 = blockIdx.y * 32, a = threadIdx.x & 31, b = threadIdx.x >> 5;
+  for (int p = b; p < 32; p += 8) {
+    const int64_t off = j0 + a + (int64_t)(p0 + p) * n;
+    if (j0 + a < n && p0 + p < npls) tile[p][a] = m2c != 0.0 ? u1[off] * m1c + u2[off] * m2c : u1[off] * m1c;
   }
-  const int64_t b = rowptr[row], e = rowptr[row + 1];
-  for (int p0 = 0; p0 < npls; p0 += 8) {
-    double v[8];
+  __syncthreads();
+  const int w = min(32, npls - p0);  // this tile's sources
+  for (int q = threadIdx.x; q < 32 * w; q += 256) {
+    const int j = q / w, p = q - j * w;
+    if (j0 + j < n) v[(int64_t)(j0 + j) * npls + p0 + p] = tile[p][j];
+  }
+}
+
+// rhs = C v + coef S for 32 rows a CTA, G lanes a row, a source per lane (32 sources at a
+// time): every entry is one contiguous read of its sources' values and there is nothing
+// to reduce; the results go through shared memory to the column-major right-hand side.
+// Bound by the reads of v through L1 and L2 (33 entries x 8 npls bytes a row).  With a
+// warp a row over column-major vectors, every one of 32 lanes gathering its own entry for
+// eight sources in turn, this was 1,885 us at 345,744 edges and 32 sources; now 287 and
+// 54 for the combination above.
+template <int G>
+__global__ void __launch_bounds__(256) k_history_rhs_multi(const int64_t* __restrict__ rowptr,
+                                                           const int* __restrict__ col, const double* __restrict__ C,
+                                                           const double* __restrict__ v,
+                                                           const double* __restrict__ S, double coef,
+                                                           const uint8_t* __restrict__ bound, int n, int npls,
+                                                           double* __restrict__ rhs) {
+  __shared__ double out[32][33];  // [source][row]
+  const int row0 = blockIdx.x * 32, sub = threadIdx.x % G, grp = threadIdx.x / G;
+  for (int p0 = 0; p0 < npls; p0 += 32) {
+    const int p = p0 + sub;
+    for (int r = grp; r < 32; r += 256 / G) {
+      const int row = row0 + r;
+      double acc[2] = {0.0, 0.0};
+      if (row < n && !bound[row] && p < npls) {
+        const int64_t b = rowptr[row], e = rowptr[row + 1];
+        int64_t q = b;
+        for (; q + 4 <= e; q += 4) {
+          int j[4];
+          double c[4], x[4];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) v[r] = 0.0;
-    for (int64_t q = b + lane; q < e; q += 32) {
-      const double c = C[q];
-      const int64_t j = col[q];
+          for (int i = 0; i < 4; ++i) j[i] = __ldg(col + q + i);
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int64_t off = j + (int64_t)(p0 + r) * n;
-        if (p0 + r < npls) v[r] = fma(c, m2c != 0.0 ? u1[off] * m1c + u2[off] * m2c : u1[off] * m1c, v[r]);
+          for (int i = 0; i < 4; ++i) {
+            c[i] = __ldg(C + q + i);
+            x[i] = __ldg(v + (int64_t)j[i] * npls + p);
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[i & 1] = fma(c[i], x[i], acc[i & 1]);
+        }
+        for (; q < e; ++q) acc[0] = fma(__ldg(C + q), __ldg(v + (int64_t)__ldg(col + q) * npls + p), acc[0]);
+      }
+      out[sub][r] = acc[0] + acc[1];
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < 32 * min(G, npls - p0); q += 256) {
+      const int r = q & 31, pp = q >> 5, row = row0 + r;
+      if (row < n) {
+        double t = out[pp][r];
+        if (coef != 0.0 && !bound[row]) t += coef * S[row + (int64_t)(p0 + pp) * n];
+        rhs[row + (int64_t)(p0 + pp) * n] = t;
       }
     }
-    double a4[4], a2[2];
-    bool up = (lane & 16) != 0;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const double mine = up ? v[4 + r] : v[r], other = up ? v[r] : v[4 + r];
-      a4[r] = mine + __shfl_xor_sync(0xffffffffu, other, 16);
-    }
-    up = (lane & 8) != 0;
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const double mine = up ? a4[2 + r] : a4[r], other = up ? a4[r] : a4[2 + r];
-      a2[r] = mine + __shfl_xor_sync(0xffffffffu, other, 8);
-    }
-    up = (lane & 4) != 0;
-    double a1 = (up ? a2[1] : a2[0]) + __shfl_xor_sync(0xffffffffu, up ? a2[0] : a2[1], 4);
-    a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
-    a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
-    if ((lane & 3) == 0) {
-      const int p = p0 + 4 * ((lane >> 4) & 1) + 2 * ((lane >> 3) & 1) + ((lane >> 2) & 1);
-      if (p < npls) {
-        double t = a1;
-        if (coef != 0.0) t += coef * S[row + (int64_t)p * n];
-        rhs[row + (int64_t)p * n] = t;
-      }
-    }
+    __syncthreads();
   }
 }
 
@@ -443,11 +455,25 @@ void launch_combine(const double* Cval, const double* Bval, const int64_t* src, 
 
 void launch_history_rhs(const int64_t* rowptr, const int* col, const double* Cval, const double* u1,
                         const double* u2, double m1c, double m2c, const double* S, double coef,
-                        const uint8_t* bound, int n, int npls, double* rhs, cudaStream_t s) {
+                        const uint8_t* bound, int n, int npls, double* rhs, double* scratch,
+                        cudaStream_t s) {
   if (npls > 1) {
-    const int64_t threads = (int64_t)n * 32;
-    k_history_rhs_multi<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(rowptr, col, Cval, u1, u2, m1c, m2c, S,
-                                                                          coef, bound, n, npls, rhs);
+    if (n <= 0) return;
+    const unsigned tiles = (unsigned)((n + 31) / 32);
+    k_history_combine<<<dim3(tiles, (unsigned)((npls + 31) / 32)), 256, 0, s>>>(u1, u2, m1c, m2c, n, npls, scratch);
+    auto go = [&](auto kernel) {
+      kernel<<<tiles, 256, 0, s>>>(rowptr, col, Cval, scratch, S, coef, bound, n, npls, rhs);
+    };
+    if (npls <= 2)
+      go(k_history_rhs_multi<2>);
+    else if (npls <= 4)
+      go(k_history_rhs_multi<4>);
+    else if (npls <= 8)
+      go(k_history_rhs_multi<8>);
+    else if (npls <= 16)
+      go(k_history_rhs_multi<16>);
+    else
+      go(k_history_rhs_multi<32>);
   } else {
     const int64_t threads = (int64_t)n * kRhsLanes;
     k_history_rhs<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(rowptr, col, Cval, u1, u2, m1c, m2c, S, coef,
