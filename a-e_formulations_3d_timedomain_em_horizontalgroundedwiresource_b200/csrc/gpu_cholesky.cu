@@ -12,7 +12,7 @@
 // front by binary search over the prefix, so one launch covers every front of a
 // level that takes part in the current panel.
 //
-// Factorization per level: zero the update blocks, extend-add the children,
+// Factorization per level: gather the children's update blocks,
 // then for each 64-wide inner panel [j0, j1): Cholesky of the diagonal block,
 // triangular solve of the rows below, rank-64 update of the rest of the kOuter-wide
 // outer panel [J0, J1); at the end of each outer panel one rank-(J1 - J0) update
@@ -69,41 +69,71 @@ __global__ void k_scatter_entries(T* __restrict__ L, const int64_t* __restrict__
     L[dst[q]] = (T)val[q];
 }
 
+// Where a front's rows stand in its children: the children of front s are
+// list[ptr[s] .. ptr[s + 1]); row i of s is row inv[inv_off[c] + i] of child c's update
+// block (-1: not among them).  The maps are increasing, as both row lists are sorted.
+struct Kids {
+  const int* ptr;
+  const int* list;
+  const int64_t* inv_off;
+  const int* inv;
+};
+
+__global__ void k_invert_rows(const int* __restrict__ parent, const int64_t* __restrict__ rel_off,
+                              const int* __restrict__ rel, const int64_t* __restrict__ inv_off,
+                              int* __restrict__ inv) {
+  const int c = blockIdx.x;
+  if (parent[c] < 0) return;
+  for (int64_t x = rel_off[c] + threadIdx.x; x < rel_off[c + 1]; x += blockDim.x)
+    inv[inv_off[c] + rel[x]] = (int)(x - rel_off[c]);
+}
+
+// Children's update blocks into their parents, one warp per parent column, 8 columns
+// per CTA: every entry of the parent's lower triangle gathers its children's entries in
+// order (a column of a child is read nearly in sequence), so an update block is written
+// once and needs no zeros first.  Bound by HBM: 8 bytes written and 8 read per child and
+// entry, where zeroing it and adding one child after another moved 56 bytes an entry for two
+// children (80^3: 35 ms a factorization, now 20).
 template <class T>
-__global__ void k_zero_u(T* __restrict__ U, Fronts f, const int* __restrict__ fronts,
-                         const int64_t* __restrict__ prefix, int count) {
+__global__ void __launch_bounds__(256) k_assemble_fronts(T* __restrict__ L, T* U, Fronts f, Kids kids,
+                                                         const int* __restrict__ fronts,
+                                                         const int64_t* __restrict__ prefix, int count) {
+  constexpr int N = 4;  // rows per lane and pass
   const int idx = find_task(prefix, count, blockIdx.x);
   const int s = fronts[idx];
   const int m = f.m[s], k = f.k[s], r = m - k;
-  const int64_t t = blockIdx.x - prefix[idx];
-  const int c0 = (int)t * kSolveRows, c1 = min(r, c0 + kSolveRows);
-  T* u = U + f.u_off[s];
-  // the lower triangle only: the updates, the extend-add and the trailing update
-  // read and write rows i >= c of column c and nothing above
-  for (int c = c0; c < c1; ++c)
-    for (int i = c + threadIdx.x; i < r; i += blockDim.x) u[i + (int64_t)c * r] = (T)0;
-}
-
-// Extend-add of the children's update blocks into their parents (one child per
-// parent per launch, so no two CTAs write the same parent element).  One warp
-// per child column, 8 columns per CTA.
-template <class T>
-__global__ void k_extend_add(T* __restrict__ L, T* __restrict__ U, Fronts f, const int* __restrict__ parent,
-                             const int64_t* __restrict__ rel_off, const int* __restrict__ rel,
-                             const int* __restrict__ kids, const int64_t* __restrict__ prefix, int count) {
-  const int idx = find_task(prefix, count, blockIdx.x);
-  const int c = kids[idx];
-  const int p = parent[c];
-  const int mc = f.m[c], kc = f.k[c], rc = mc - kc;
-  const int mp = f.m[p], kp = f.k[p];
-  const int64_t lo = f.l_off[p], uo = f.u_off[p];
-  const int* rl = rel + rel_off[c];
-  const T* uc = U + f.u_off[c];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = (int)(blockIdx.x - prefix[idx]) * 8 + warp;
-  if (b >= rc) return;
-  const int pc = rl[b];
-  for (int a = b + lane; a < rc; a += 32) *felem(L, U, lo, uo, mp, kp, rl[a], pc) += uc[a + (int64_t)b * rc];
+  const int c = (int)(blockIdx.x - prefix[idx]) * 8 + warp;
+  if (c >= m) return;
+  const int q0 = kids.ptr[s], q1 = kids.ptr[s + 1];
+  const bool pivot = c < k;
+  if (pivot) {  // pivot columns only change where a child reaches them
+    bool any = false;
+    for (int q = q0; q < q1; ++q) any = any || kids.inv[kids.inv_off[kids.list[q]] + c] >= 0;
+    if (!any) return;
+  }
+  T* dst = pivot ? L + f.l_off[s] + (int64_t)c * m : U + f.u_off[s] + (int64_t)(c - k) * r - k;
+  for (int i0 = c + lane; i0 < m; i0 += 32 * N) {
+    T v[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) v[e] = (pivot && i0 + 32 * e < m) ? dst[i0 + 32 * e] : (T)0;
+    for (int q = q0; q < q1; ++q) {
+      const int ch = kids.list[q];
+      const int* inv = kids.inv + kids.inv_off[ch];
+      const int b = inv[c];
+      if (b < 0) continue;
+      const T* src = U + f.u_off[ch] + (int64_t)b * (f.m[ch] - f.k[ch]);
+      int a[N];
+#pragma unroll
+      for (int e = 0; e < N; ++e) a[e] = i0 + 32 * e < m ? inv[i0 + 32 * e] : -1;
+#pragma unroll
+      for (int e = 0; e < N; ++e)
+        if (a[e] >= 0) v[e] += src[a[e]];
+    }
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      if (i0 + 32 * e < m) dst[i0 + 32 * e] = v[e];
+  }
 }
 
 __device__ __forceinline__ void dmma16816(double (&c)[4], const double (&a)[8], const double (&b)[4]) {
@@ -817,9 +847,13 @@ struct SolveArgs {
   int64_t ld;
 };
 
+// Front vectors of a level: the right-hand side on the pivot rows plus what the children
+// left on the front's rows, gathered in child order (one launch where setting up and
+// adding one child after another was three).
 template <class T>
-__global__ void k_fwd_init(T* __restrict__ W, const double* __restrict__ b, SolveArgs a,
-                           const int* __restrict__ fronts, const int64_t* __restrict__ prefix, int count) {
+__global__ void k_fwd_gather(T* W, const double* __restrict__ b, SolveArgs a, Kids kids,
+                             const int* __restrict__ fronts, const int64_t* __restrict__ prefix, int count) {
+  constexpr int N = 4;  // right-hand sides per pass
   const int idx = find_task(prefix, count, blockIdx.x);
   const int s = fronts[idx];
   const int m = a.m[s], k = a.k[s];
@@ -827,22 +861,23 @@ __global__ void k_fwd_init(T* __restrict__ W, const double* __restrict__ b, Solv
   if (i >= m) return;
   T* w = W + a.w_off[s] * a.nrhs;
   const int pos = (i < k) ? a.rows[a.rows_off[s] + i] : -1;
-  for (int r = 0; r < a.nrhs; ++r) w[i + (int64_t)r * m] = (i < k) ? (T)b[pos + r * a.ld] : (T)0;
-}
-
-template <class T>
-__global__ void k_fwd_extend(T* __restrict__ W, SolveArgs a, const int* __restrict__ parent,
-                             const int64_t* __restrict__ rel_off, const int* __restrict__ rel,
-                             const int* __restrict__ kids, const int64_t* __restrict__ prefix, int count) {
-  const int idx = find_task(prefix, count, blockIdx.x);
-  const int c = kids[idx], p = parent[c];
-  const int mc = a.m[c], kc = a.k[c], rc = mc - kc, mp = a.m[p];
-  const int i = (int)(blockIdx.x - prefix[idx]) * kSolveRows + threadIdx.x;
-  if (i >= rc) return;
-  const T* wc = W + a.w_off[c] * a.nrhs;
-  T* wp = W + a.w_off[p] * a.nrhs;
-  const int pr = rel[rel_off[c] + i];
-  for (int r = 0; r < a.nrhs; ++r) wp[pr + (int64_t)r * mp] += wc[kc + i + (int64_t)r * mc];
+  const int q0 = kids.ptr[s], q1 = kids.ptr[s + 1];
+  for (int r0 = 0; r0 < a.nrhs; r0 += N) {
+    T v[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) v[e] = (i < k && r0 + e < a.nrhs) ? (T)b[pos + (r0 + e) * a.ld] : (T)0;
+    for (int q = q0; q < q1; ++q) {
+      const int c = kids.list[q], mc = a.m[c], x = kids.inv[kids.inv_off[c] + i];
+      if (x < 0) continue;
+      const T* wc = W + a.w_off[c] * a.nrhs + a.k[c] + x;
+#pragma unroll
+      for (int e = 0; e < N; ++e)
+        if (r0 + e < a.nrhs) v[e] += wc[(int64_t)(r0 + e) * mc];
+    }
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      if (r0 + e < a.nrhs) w[i + (int64_t)(r0 + e) * m] = v[e];
+  }
 }
 
 // Forward diagonal-block solve of panel [j0, j0 + w) (one CTA per front).
@@ -2497,8 +2532,7 @@ struct LookAhead {
 
 template <class T>
 int launch_factor(const Symbolic& sy, T* L, T* U, const double* vals, const int64_t* entry, Fronts fr,
-                  const int* parent, const int64_t* rel_off, const int* rel, const int* tasks,
-                  const int64_t* prefix, int* err, const int* c0, bool use_tc, cudaStream_t s,
+                  const Kids& kids, const int* tasks, const int64_t* prefix, int* err, const int* c0, bool use_tc, cudaStream_t s,
                   const OzakiBuffers* oz = nullptr, const int64_t* aux = nullptr,
                   std::vector<cudaEvent_t>* oz_ev = nullptr, size_t* oz_used = nullptr, T* dinv = nullptr,
                   const int64_t* dinv_off = nullptr, const LookAhead* la = nullptr) {
@@ -2516,15 +2550,10 @@ int launch_factor(const Symbolic& sy, T* L, T* U, const double* vals, const int6
     }
   }
   for (const LevelPlan& lp : sy.levels) {
-    if (lp.assemble.ctas > 0) {
-      k_zero_u<T><<<grid_of(lp.assemble.ctas), 256, 0, s>>>(U, fr, tasks + lp.assemble.off, prefix + lp.assemble.pre,
-                                                           lp.assemble.count);
-      ++launches;
-    }
-    for (const TaskList& tl : lp.extend_slots) {
-      if (tl.ctas == 0) continue;
-      k_extend_add<T><<<grid_of(tl.ctas), 256, 0, s>>>(L, U, fr, parent, rel_off, rel, tasks + tl.off,
-                                                       prefix + tl.pre, tl.count);
+    if (lp.assemble_cols.ctas > 0) {
+      k_assemble_fronts<T><<<grid_of(lp.assemble_cols.ctas), 256, 0, s>>>(L, U, fr, kids, tasks + lp.assemble_cols.off,
+                                                                          prefix + lp.assemble_cols.pre,
+                                                                          lp.assemble_cols.count);
       ++launches;
     }
     for (const PanelStep& ps : lp.panels) {
@@ -2621,20 +2650,14 @@ int launch_factor(const Symbolic& sy, T* L, T* U, const double* vals, const int6
 
 template <class T>
 int launch_solve(const Symbolic& sy, const T* L, T* W, T* part, const double* b, double* x, SolveArgs a,
-                 const int* parent, const int64_t* rel_off, const int* rel, const int* tasks, const int64_t* prefix,
+                 const Kids& kids, const int* tasks, const int64_t* prefix,
                  cudaStream_t s) {
   int launches = 0;
   const size_t ysm = sizeof(T) * P * a.nrhs;
   for (const LevelPlan& lp : sy.levels) {
-    k_fwd_init<T><<<grid_of(lp.assemble.ctas), kSolveRows, 0, s>>>(W, b, a, tasks + lp.assemble.off,
-                                                                   prefix + lp.assemble.pre, lp.assemble.count);
+    k_fwd_gather<T><<<grid_of(lp.assemble.ctas), kSolveRows, 0, s>>>(W, b, a, kids, tasks + lp.assemble.off,
+                                                                     prefix + lp.assemble.pre, lp.assemble.count);
     ++launches;
-    for (const TaskList& tl : lp.extend_vec) {
-      if (tl.ctas == 0) continue;
-      k_fwd_extend<T><<<grid_of(tl.ctas), kSolveRows, 0, s>>>(W, a, parent, rel_off, rel, tasks + tl.off,
-                                                              prefix + tl.pre, tl.count);
-      ++launches;
-    }
     for (const PanelStep& ps : lp.panels) {
       k_fwd_diag<T><<<ps.potrf.count, 256, ysm, s>>>(L, W, a, tasks + ps.potrf.off, ps.j0);
       ++launches;
@@ -2675,7 +2698,7 @@ int launch_solve(const Symbolic& sy, const T* L, T* W, T* part, const double* b,
 // sides per thread.
 template <class T, int RPT, bool STREAM, bool MR = false>
 void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T* part, const double* b, double* x,
-                         SolveArgs a, const int* parent, const int64_t* rel_off, const int* rel, const int* tasks,
+                         SolveArgs a, const Kids& kids, const int* tasks,
                          const int64_t* prefix, FusedArgs fa, int* sync, const int (&resident)[2], int& launches,
                          cudaStream_t s) {
   static_assert(!MR || std::is_same<T, double>::value, "the many-column persistent kernels are FP64");
@@ -2691,15 +2714,9 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
   };
   for (int l = 0; l < nlev; ++l) {
     const LevelPlan& lp = sy.levels[l];
-    k_fwd_init<T><<<grid_of(lp.assemble.ctas), kSolveRows, 0, s>>>(W, b, a, tasks + lp.assemble.off,
-                                                                   prefix + lp.assemble.pre, lp.assemble.count);
+    k_fwd_gather<T><<<grid_of(lp.assemble.ctas), kSolveRows, 0, s>>>(W, b, a, kids, tasks + lp.assemble.off,
+                                                                     prefix + lp.assemble.pre, lp.assemble.count);
     ++launches;
-    for (const TaskList& tl : lp.extend_vec) {
-      if (tl.ctas == 0) continue;
-      k_fwd_extend<T><<<grid_of(tl.ctas), kSolveRows, 0, s>>>(W, a, parent, rel_off, rel, tasks + tl.off,
-                                                              prefix + tl.pre, tl.count);
-      ++launches;
-    }
     if (lp.fwd_count == 0) continue;
     FusedArgs f = fa;
     f.units = fa.units + (int64_t)kUnitInts * lp.fwd_off;
@@ -2737,11 +2754,11 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
 
 template <class T>
 int launch_solve_fused(const Symbolic& sy, const T* L, const T* Dinv, T* W, T* part, const double* b, double* x,
-                       SolveArgs a, const int* parent, const int64_t* rel_off, const int* rel, const int* tasks,
+                       SolveArgs a, const Kids& kids, const int* tasks,
                        const int64_t* prefix, FusedArgs fa, int* sync, const int (&resident)[2][2], cudaStream_t s) {
   int launches = 0;
 #define TDEM_LEVELS(R, ST, RES) \
-  launch_level_solves<T, R, ST>(sy, L, Dinv, W, part, b, x, a, parent, rel_off, rel, tasks, prefix, fa, sync, RES, \
+  launch_level_solves<T, R, ST>(sy, L, Dinv, W, part, b, x, a, kids, tasks, prefix, fa, sync, RES, \
                                 launches, s)
   if (a.nrhs == 1)
     TDEM_LEVELS(1, true, resident[0]);
@@ -2763,12 +2780,11 @@ int launch_solve_fused(const Symbolic& sy, const T* L, const T* Dinv, T* W, T* p
 
 // The persistent many-column level solves (FP64, 3 <= nrhs <= 32).
 int launch_solve_mr(const Symbolic& sy, const double* L, const double* Dinv, double* W, double* part, const double* b,
-                    double* x, SolveArgs a, const int* parent, const int64_t* rel_off, const int* rel,
-                    const int* tasks, const int64_t* prefix, FusedArgs fa, int* sync, const int (&resident)[2],
+                    double* x, SolveArgs a, const Kids& kids, const int* tasks, const int64_t* prefix, FusedArgs fa, int* sync, const int (&resident)[2],
                     cudaStream_t s) {
   int launches = 0;
 #define TDEM_MR(R) \
-  launch_level_solves<double, R, false, true>(sy, L, Dinv, W, part, b, x, a, parent, rel_off, rel, tasks, prefix, \
+  launch_level_solves<double, R, false, true>(sy, L, Dinv, W, part, b, x, a, kids, tasks, prefix, \
                                               fa, sync, resident, launches, s)
   if (a.nrhs <= 4)
     TDEM_MR(1);
@@ -2890,6 +2906,7 @@ int64_t GpuCholesky::bytes_needed(const Symbolic& sy, int nrhs_max, int precisio
   if (fel != el) b += slot_bytes(sy, (int)fel);  // the FP64 work factor of a demoted setup
   if (fel == 8) b += sy.oz_rows_max * ((int64_t)kOzModuli * kOzK + 4);  // residues + exponents
   b += 8 * (int64_t)sy.task_aux.size();
+  b += 4 * sy.kid_rows + 8 * (int64_t)sy.front_m.size();  // child maps
   b += 8 * (int64_t)(sy.l_off.size() + sy.u_off.size() + sy.wvec_off.size() + sy.entry_dst.size() +
                      sy.rel_off.size() + sy.rows_off.size() + sy.task_prefix.size() + sy.dinv_off.size());
   b += 4 * (int64_t)(sy.front_m.size() + sy.front_k.size() + sy.rel.size() + sy.rows_all.size() + sy.tasks.size() +
@@ -2927,8 +2944,6 @@ std::string GpuCholesky::setup(Symbolic&& sy, const std::vector<int>& perm_to_ve
   if (!(e = upload(&d_m_, sy_.front_m, s)).empty()) return e;
   if (!(e = upload(&d_k_, sy_.front_k, s)).empty()) return e;
   if (!(e = upload(&d_entry_, sy_.entry_dst, s)).empty()) return e;
-  if (!(e = upload(&d_rel_off_, sy_.rel_off, s)).empty()) return e;
-  if (!(e = upload(&d_rel_, sy_.rel, s)).empty()) return e;
   if (!(e = upload(&d_rows_off_, sy_.rows_off, s)).empty()) return e;
   {
     std::vector<int> rows(sy_.rows_all.size());
@@ -2944,7 +2959,7 @@ std::string GpuCholesky::setup(Symbolic&& sy, const std::vector<int>& perm_to_ve
     if (!(e = alloc((void**)&oz_.exps, sizeof(int) * (size_t)oz_.rows)).empty()) return e;
     if (!(e = ozaki_setup(oz_)).empty()) return e;
   }
-  if (!(e = upload(&d_parent_, sy_.front_parent, s)).empty()) return e;
+  if (!(e = setup_kids(s)).empty()) return e;
   if (!(e = upload(&d_c0_, sy_.front_c0, s)).empty()) return e;
   if (!(e = upload(&d_items_, sy_.solve_items, s)).empty()) return e;
   if (!(e = upload(&d_dinv_off_, sy_.dinv_off, s)).empty()) return e;
@@ -2964,6 +2979,44 @@ std::string GpuCholesky::setup(Symbolic&& sy, const std::vector<int>& perm_to_ve
     return e;
   if (elem_ == 8 && !(e = mr_residency(resident_mr_, sms_)).empty()) return e;
   TDEM_CUDA_TRY(cudaStreamSynchronize(s));
+  return "";
+}
+
+// The fronts' children and the maps of their rows into the children (Kids), turned on the
+// device from the child-to-parent maps of the analysis.
+std::string GpuCholesky::setup_kids(cudaStream_t s) {
+  const int nf = (int)sy_.fronts.size();
+  std::vector<int> ptr(nf + 1, 0), list;
+  std::vector<int64_t> inv_off(nf, 0);
+  int64_t total = 0;
+  for (int f = 0; f < nf; ++f) {
+    for (int c : sy_.fronts[f].children) {
+      list.push_back(c);
+      inv_off[c] = total;
+      total += sy_.front_m[f];
+    }
+    ptr[f + 1] = (int)list.size();
+  }
+  std::string e;
+  int *parent = nullptr, *rel = nullptr;
+  int64_t* rel_off = nullptr;
+  if (!(e = upload(&d_kid_ptr_, ptr, s)).empty()) return e;
+  if (!(e = upload(&d_kid_list_, list, s)).empty()) return e;
+  if (!(e = upload(&d_inv_off_, inv_off, s)).empty()) return e;
+  if (!(e = alloc((void**)&d_inv_, sizeof(int) * (size_t)std::max<int64_t>(1, total))).empty()) return e;
+  const size_t kept = allocs_.size(), kept_bytes = bytes_;
+  if (!(e = upload(&parent, sy_.front_parent, s)).empty()) return e;
+  if (!(e = upload(&rel_off, sy_.rel_off, s)).empty()) return e;
+  if (!(e = upload(&rel, sy_.rel, s)).empty()) return e;
+  TDEM_CUDA_TRY(cudaMemsetAsync(d_inv_, 0xFF, sizeof(int) * (size_t)std::max<int64_t>(1, total), s));
+  if (nf > 0) k_invert_rows<<<(unsigned)nf, 256, 0, s>>>(parent, rel_off, rel, d_inv_off_, d_inv_);
+  TDEM_CUDA_TRY(cudaGetLastError());
+  TDEM_CUDA_TRY(cudaStreamSynchronize(s));
+  while (allocs_.size() > kept) {  // the child-to-parent maps are done with
+    cudaFree(allocs_.back());
+    allocs_.pop_back();
+  }
+  bytes_ = kept_bytes;
   return "";
 }
 
@@ -2992,6 +3045,7 @@ bool GpuCholesky::lookahead_ready(cudaStream_t s) {
 }
 
 void GpuCholesky::factor(const double* d_vals, cudaStream_t s, int slot) {
+  const Kids kids{d_kid_ptr_, d_kid_list_, d_inv_off_, d_inv_};
   Fronts fr{d_l_off_, d_u_off_, d_m_, d_k_};
   LookAhead la;
   if (elem_ == 8 || demoted()) {
@@ -3008,8 +3062,7 @@ void GpuCholesky::factor(const double* d_vals, cudaStream_t s, int slot) {
   void* Dp = d_dinv_[slot];
   if (demoted()) {
     // FP64 factorization into the work factor, then both arrays rounded into the slot
-    launches_factor_ = launch_factor<double>(sy_, (double*)d_Lw_, (double*)d_U_, d_vals, d_entry_, fr, d_parent_,
-                                             d_rel_off_, d_rel_, d_tasks_, d_prefix_, d_err_, d_c0_, false, s,
+    launches_factor_ = launch_factor<double>(sy_, (double*)d_Lw_, (double*)d_U_, d_vals, d_entry_, fr, kids, d_tasks_, d_prefix_, d_err_, d_c0_, false, s,
                                              ozaki() ? &oz_ : nullptr, d_task_aux_,
                                              oz_timing_ ? &oz_events_ : nullptr, &oz_used_, (double*)d_dinvw_,
                                              d_dinv_off_, &la);
@@ -3022,13 +3075,11 @@ void GpuCholesky::factor(const double* d_vals, cudaStream_t s, int slot) {
     return;
   }
   if (elem_ == 4) {
-    launches_factor_ = launch_factor<float>(sy_, (float*)Lp, (float*)d_U_, d_vals, d_entry_, fr, d_parent_,
-                                            d_rel_off_, d_rel_, d_tasks_, d_prefix_, d_err_, d_c0_, tc_update_, s);
+    launches_factor_ = launch_factor<float>(sy_, (float*)Lp, (float*)d_U_, d_vals, d_entry_, fr, kids, d_tasks_, d_prefix_, d_err_, d_c0_, tc_update_, s);
     if (ni) k_diag_inverse<float><<<ni, 256, ism, s>>>((const float*)Lp, (float*)Dp, fr, d_dinv_off_,
                                                        d_items_ + 2 * sy_.inv_off);
   } else {
-    launches_factor_ = launch_factor<double>(sy_, (double*)Lp, (double*)d_U_, d_vals, d_entry_, fr, d_parent_,
-                                             d_rel_off_, d_rel_, d_tasks_, d_prefix_, d_err_, d_c0_, false, s,
+    launches_factor_ = launch_factor<double>(sy_, (double*)Lp, (double*)d_U_, d_vals, d_entry_, fr, kids, d_tasks_, d_prefix_, d_err_, d_c0_, false, s,
                                              ozaki() ? &oz_ : nullptr, d_task_aux_,
                                              oz_timing_ ? &oz_events_ : nullptr, &oz_used_, (double*)Dp,
                                              d_dinv_off_, &la);
@@ -3055,6 +3106,7 @@ void GpuCholesky::solve(const double* d_b, double* d_x, int64_t ld, int nrhs, cu
 
 void GpuCholesky::solve_with(const SolveSchedule& sc, const double* d_b, double* d_x, int64_t ld, int nrhs,
                              cudaStream_t s, int slot) {
+  const Kids kids{d_kid_ptr_, d_kid_list_, d_inv_off_, d_inv_};
   if (sc.split > 1 && nrhs > 1) {
     // column groups one after another (each its own complete solve)
     const int per = (nrhs + sc.split - 1) / sc.split;
@@ -3077,7 +3129,7 @@ void GpuCholesky::solve_with(const SolveSchedule& sc, const double* d_b, double*
     for (int d = 0; d < 2; ++d)
       res[d] = solve_ctas_cap_ > 0 ? std::min(resident_mr_[d], solve_ctas_cap_ * sms_) : resident_mr_[d];
     launches_solve_ = launch_solve_mr(sy_, (const double*)Lp, (const double*)Dp, (double*)d_W_, (double*)d_spart_,
-                                      d_b, d_x, a, d_parent_, d_rel_off_, d_rel_, d_tasks_, d_prefix_, fa, d_sync_,
+                                      d_b, d_x, a, kids, d_tasks_, d_prefix_, fa, d_sync_,
                                       res, s);
     return;
   }
@@ -3089,20 +3141,18 @@ void GpuCholesky::solve_with(const SolveSchedule& sc, const double* d_b, double*
         res[j][d] = solve_ctas_cap_ > 0 ? std::min(resident_[j][d], solve_ctas_cap_ * sms_) : resident_[j][d];
     if (elem_ == 4)
       launches_solve_ = launch_solve_fused<float>(sy_, (const float*)Lp, (const float*)Dp, (float*)d_W_,
-                                                  (float*)d_spart_, d_b, d_x, a, d_parent_, d_rel_off_, d_rel_,
-                                                  d_tasks_, d_prefix_, fa, d_sync_, res, s);
+                                                  (float*)d_spart_, d_b, d_x, a, kids, d_tasks_, d_prefix_, fa, d_sync_, res, s);
     else
       launches_solve_ = launch_solve_fused<double>(sy_, (const double*)Lp, (const double*)Dp, (double*)d_W_,
-                                                   (double*)d_spart_, d_b, d_x, a, d_parent_, d_rel_off_, d_rel_,
-                                                   d_tasks_, d_prefix_, fa, d_sync_, res, s);
+                                                   (double*)d_spart_, d_b, d_x, a, kids, d_tasks_, d_prefix_, fa, d_sync_, res, s);
     return;
   }
   if (elem_ == 4)
     launches_solve_ = launch_solve<float>(sy_, (const float*)Lp, (float*)d_W_, (float*)d_part_, d_b, d_x, a,
-                                          d_parent_, d_rel_off_, d_rel_, d_tasks_, d_prefix_, s);
+                                          kids, d_tasks_, d_prefix_, s);
   else
     launches_solve_ = launch_solve<double>(sy_, (const double*)Lp, (double*)d_W_, (double*)d_part_, d_b, d_x, a,
-                                           d_parent_, d_rel_off_, d_rel_, d_tasks_, d_prefix_, s);
+                                           kids, d_tasks_, d_prefix_, s);
 }
 
 // Times every candidate schedule for nrhs columns on the factor in `slot` (stream

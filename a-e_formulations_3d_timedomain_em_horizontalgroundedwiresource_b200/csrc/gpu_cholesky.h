@@ -182,13 +182,15 @@ class GpuCholesky {
   int* d_m_ = nullptr;
   int* d_k_ = nullptr;
   int64_t* d_entry_ = nullptr;
-  int64_t* d_rel_off_ = nullptr;
-  int* d_rel_ = nullptr;
+  int* d_kid_ptr_ = nullptr;     // the fronts' children and row maps (Kids in gpu_cholesky.cu)
+  int* d_kid_list_ = nullptr;
+  int64_t* d_inv_off_ = nullptr;
+  int* d_inv_ = nullptr;
+  std::string setup_kids(cudaStream_t s);
   int64_t* d_rows_off_ = nullptr;
   int* d_rows_ = nullptr;        // rows_all mapped to caller vector positions
   int* d_tasks_ = nullptr;
   int64_t* d_prefix_ = nullptr;
-  int* d_parent_ = nullptr;
   int* d_c0_ = nullptr;
   int* d_err_ = nullptr;         // [0] first non-positive pivot, [1] level-solve wait gave up,
                                  // [2] tensor-core update wait gave up

@@ -655,32 +655,15 @@ std::string analyse(int n, const int64_t* rowptr, const int* colind, const doubl
   int64_t max_partials = 0;
   for (int l = 0; l < nlev; ++l) {
     LevelPlan& lp = sy.levels[l];
-    // extend-add slots: slot j = j-th child of each front at this level; one CTA
-    // per child column block of 8 columns
-    int max_kids = 0;
-    for (int s : lp.fronts) max_kids = std::max(max_kids, (int)sy.fronts[s].children.size());
-    for (int j = 0; j < max_kids; ++j) {
-      std::vector<int> fr;
-      std::vector<int64_t> ct, cv;
-      for (int s : lp.fronts)
-        if ((int)sy.fronts[s].children.size() > j) {
-          const int ch = sy.fronts[s].children[j];
-          const int64_t r = (int64_t)sy.fronts[ch].rows.size();
-          if (r == 0) continue;
-          fr.push_back(ch);
-          ct.push_back(cdiv(r, 8));
-          cv.push_back(cdiv(r, kSolveRows));
-        }
-      TaskList tl, tv;
-      add_tasks(sy, tl, fr, ct);
-      add_tasks(sy, tv, fr, cv);
-      lp.extend_slots.push_back(tl);
-      lp.extend_vec.push_back(tv);
-    }
     {
-      std::vector<int64_t> ct;
-      for (int s : lp.fronts) ct.push_back(cdiv(sy.front_m[s], kSolveRows));
+      std::vector<int64_t> ct, cc;
+      for (int s : lp.fronts) {
+        ct.push_back(cdiv(sy.front_m[s], kSolveRows));
+        cc.push_back(cdiv(sy.front_m[s], 8));
+        sy.kid_rows += (int64_t)sy.fronts[s].children.size() * sy.front_m[s];
+      }
       add_tasks(sy, lp.assemble, lp.fronts, ct);
+      add_tasks(sy, lp.assemble_cols, lp.fronts, cc);
     }
     int kmax = 0;
     for (int s : lp.fronts) kmax = std::max(kmax, sy.front_k[s]);

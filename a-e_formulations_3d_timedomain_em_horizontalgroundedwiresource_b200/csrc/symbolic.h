@@ -11,7 +11,7 @@
 //
 // Everything the numeric phase needs on the device is flattened here:
 //   * front offsets / sizes, entry map (matrix value -> front slot),
-//   * child -> parent relative row maps for extend-add,
+//   * child -> parent relative row maps of the assembly,
 //   * per-level, per-panel task lists for the batched dense kernels,
 //   * per-front row index lists for the triangular solves.
 #pragma once
@@ -100,9 +100,8 @@ struct PanelStep {
 
 struct LevelPlan {
   std::vector<int> fronts;             // fronts at this height
-  std::vector<TaskList> extend_slots;  // extend-add launches (one per child slot), 8 columns per CTA
-  std::vector<TaskList> extend_vec;    // solve extend-add per child slot, kSolveRows rows per CTA
-  TaskList assemble;                   // solve: front-vector init, ceil(m / kSolveRows) CTAs each
+  TaskList assemble;                   // solve: front vectors, ceil(m / kSolveRows) CTAs each
+  TaskList assemble_cols;              // factorization: children's blocks, ceil(m / 8) CTAs each
   std::vector<PanelStep> panels;
   // Level triangular solves: units (kUnitInts ints each, see Symbolic::solve_units)
   // at solve_units[kUnitInts * off ...], taken by CTAs in list (ticket) order.
@@ -130,6 +129,7 @@ struct Symbolic {
   std::vector<int64_t> entry_dst;    // lower-CSR entry q -> offset in L
   std::vector<int64_t> rel_off;      // per front: offset of its rel map (rows -> parent slot)
   std::vector<int> rel;              // concatenated rel maps
+  int64_t kid_rows = 0;              // sum over children of their parent's m (inverse row maps)
   std::vector<int64_t> rows_off;     // per front: offset of its full row list (k + r entries)
   std::vector<int> rows_all;         // concatenated [c0..c1) U rows, permuted numbering
   std::vector<int64_t> wvec_off;     // per front: offset of its m-long solve vector
