@@ -1244,6 +1244,21 @@ __device__ __forceinline__ void store_acc(const double (&acc)[NTW][4], double* O
   }
 }
 
+// f(row, r, value) for every MMA accumulator this thread holds
+template <int NTW, class F>
+__device__ __forceinline__ void for_acc(const double (&acc)[NTW][4], int ntiles, F&& f) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+  const int mt = warp & 3;
+#pragma unroll
+  for (int j = 0; j < NTW; ++j) {
+    const int nt = (warp >> 2) + 2 * j;
+    if (nt < ntiles) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) f(16 * mt + g + 8 * (i >> 1), 8 * nt + 2 * q + (i & 1), acc[j][i]);
+    }
+  }
+}
+
 // Forward unit (many right-hand sides): row block R of front s (R < pb: pivot rows
 // [64R, ..); else update rows [k + 64 (R - pb), ..)), accumulating L_Rq y_q for
 // the pivot blocks q in [lo, hi).  Chunk units publish partial sums; the final
@@ -2041,9 +2056,10 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
 // unit whose inputs are all solved (every unit except a chain link caught before
 // its newest block is ready) waits once and prefetches solution blocks as well;
 // a chain link waits per block and reads that block's solution values directly.
-// Diagonal inverses of final pivot units are held in registers from the start.
-// Results are bitwise those of k_fwd_level / k_bwd_level (same products in the
-// same order).
+// Diagonal inverses of final pivot units are held in registers from the start and
+// applied on the FP64 tensor pipe like the blocks (as 64 multiply-adds per value on the
+// CUDA cores, each with its own shared-memory operand, they were half of a chain link).
+// Products and sums are those of k_fwd_level / k_bwd_level but for the inverses' order.
 // ---------------------------------------------------------------------------
 constexpr int kMrStages = 2;
 constexpr int kMrYld = ys_ld(32);  // solution-block stage leading dimension (32 columns)
@@ -2216,31 +2232,22 @@ __global__ void __launch_bounds__(256, 2) k_fwd_mrhs(const double* __restrict__ 
         const int r = g + 4 * j;
         if (r < nr_rhs) Zs[i * ysl + r] = (i < nr) ? wrow[j] - (tot[j] + acc[j]) : 0.0;
       }
+      for (int r = nr_rhs + g; r < 8 * ntl; r += 4) Zs[i * ysl + r] = 0.0;
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
         const int q = t + 256 * e;
         Ds[q >> 6][q & 63] = dpre[e];
       }
       __syncthreads();
-      double y[RPT];
+      double y[NTW][4];
 #pragma unroll
-      for (int j = 0; j < RPT; ++j) y[j] = 0.0;
-#pragma unroll 8
-      for (int c = 0; c < SB; ++c) {
-        const double l = Ds[c][i];
+      for (int j = 0; j < NTW; ++j)
 #pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-          const int r = g + 4 * j;
-          if (r < nr_rhs) y[j] = fma(l, Zs[c * ysl + r], y[j]);
-        }
-      }
-      if (i < nr) {
-#pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-          const int r = g + 4 * j;
-          if (r < nr_rhs) w[r0 + i + (int64_t)r * m] = y[j];
-        }
-      }
+        for (int e = 0; e < 4; ++e) y[j][e] = 0.0;
+      block_dmma<false, NTW>(y, Ds, Zs, ysl, ntl);
+      for_acc<NTW>(y, ntl, [&](int row, int r, double v) {
+        if (row < nr && r < nr_rhs) w[r0 + row + (int64_t)r * m] = v;
+      });
     }
     const bool publish = !fin || piv;
     if (t == 0) s_tk[par ^ 1] = next;
@@ -2393,35 +2400,25 @@ __global__ void __launch_bounds__(256, 2) k_bwd_mrhs(const double* __restrict__ 
         const int r = g + 4 * j;
         if (r < nr_rhs) Zs[c * ysl + r] = (c < wc) ? wrow[j] - (tot[j] + acc[j]) : 0.0;
       }
+      for (int r = nr_rhs + g; r < 8 * ntl; r += 4) Zs[c * ysl + r] = 0.0;
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
         const int q = t + 256 * e;
         Ds[q >> 6][q & 63] = dpre[e];
       }
       __syncthreads();
-      double xv[RPT];
+      double xv[NTW][4];
 #pragma unroll
-      for (int j = 0; j < RPT; ++j) xv[j] = 0.0;
-#pragma unroll 8
-      for (int ii = 0; ii < SB; ++ii) {
-        const double l = Ds[c][ii];
+      for (int j = 0; j < NTW; ++j)
 #pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-          const int r = g + 4 * j;
-          if (r < nr_rhs) xv[j] = fma(l, Zs[ii * ysl + r], xv[j]);
+        for (int e = 0; e < 4; ++e) xv[j][e] = 0.0;
+      block_dmma<true, NTW>(xv, Ds, Zs, ysl, ntl);
+      for_acc<NTW>(xv, ntl, [&](int row, int r, double v) {
+        if (row < wc && r < nr_rhs) {
+          w[c0 + row + (int64_t)r * m] = v;
+          x[rows[u.w_off + c0 + row] + (int64_t)r * ldx] = v;
         }
-      }
-      if (c < wc) {
-        const int pos = rows[u.w_off + c0 + c];
-#pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-          const int r = g + 4 * j;
-          if (r < nr_rhs) {
-            w[c0 + c + (int64_t)r * m] = xv[j];
-            x[pos + (int64_t)r * ldx] = xv[j];
-          }
-        }
-      }
+      });
     }
     if (t == 0) s_tk[par ^ 1] = next;
     __syncthreads();
