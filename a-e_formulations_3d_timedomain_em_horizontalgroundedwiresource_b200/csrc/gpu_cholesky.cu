@@ -47,6 +47,30 @@ struct Fronts {
   const int* k;
 };
 
+// Programmatic dependent launches: a kernel launched by launch_next may start while its
+// predecessor in the stream still runs, and reads or writes nothing the predecessor (or
+// what came before it) touches until wait_previous returns, which is when the
+// predecessor's grid has ended and its writes are visible; next_may_start says when the
+// successor may be set up.  What is saved is the launch and the ramp between dependent
+// kernels of a few microseconds, of which a time step of a small mesh has dozens.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+void launch_next(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Element (i, c), i >= c, of a split front.
 template <class T>
 __device__ __forceinline__ T* felem(T* L, T* U, int64_t lo, int64_t uo, int m, int k, int i, int c) {
@@ -854,6 +878,8 @@ template <class T>
 __global__ void k_fwd_gather(T* W, const double* __restrict__ b, SolveArgs a, Kids kids,
                              const int* __restrict__ fronts, const int64_t* __restrict__ prefix, int count) {
   constexpr int N = 4;  // right-hand sides per pass
+  next_may_start();
+  wait_previous();
   const int idx = find_task(prefix, count, blockIdx.x);
   const int s = fronts[idx];
   const int m = a.m[s], k = a.k[s];
@@ -948,6 +974,8 @@ __global__ void __launch_bounds__(kSolveRows) k_fwd_update(const T* __restrict__
 template <class T>
 __global__ void k_bwd_init(T* __restrict__ W, const double* __restrict__ x, SolveArgs a,
                            const int* __restrict__ fronts, const int64_t* __restrict__ prefix, int count) {
+  next_may_start();
+  wait_previous();
   const int idx = find_task(prefix, count, blockIdx.x);
   const int s = fronts[idx];
   const int m = a.m[s], k = a.k[s];
@@ -1278,6 +1306,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_level(const T* __restrict__ L, c
   constexpr bool kMma = std::is_same<T, double>::value;
   constexpr int NTW = (RPT + 3) / 4;  // column tiles per warp (nrhs <= 4 RPT)
   const int t = threadIdx.x, i = t & 63, g = t >> 6;
+  wait_previous();
   if (t == 0) s_item = atomicAdd(fa.ticket, 1);
   __syncthreads();
   const Unit u = load_unit(fa.units, s_item);
@@ -1439,6 +1468,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_level(const T* __restrict__ L, c
   constexpr bool kMma = std::is_same<T, double>::value;
   constexpr int NTW = (RPT + 3) / 4;
   const int t = threadIdx.x, c = t & 63, g = t >> 6;
+  wait_previous();
   if (t == 0) s_item = atomicAdd(fa.ticket, 1);
   __syncthreads();
   const Unit u = load_unit(fa.units, s_item);
@@ -1688,6 +1718,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
   const int t = threadIdx.x, i = t & 63, g = t >> 6, lane = t & 31;
   if (t == 0) s_tk[0] = atomicAdd(fa.ticket, 1);
   __syncthreads();
+  bool started = false;
   for (int par = 0;; par ^= 1) {
     const int tk = s_tk[par];
     if (tk >= fa.count) break;
@@ -1710,6 +1741,10 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
       const int q = lo + j;
       if (q < hi) cp_block(stage + j * SB * SB, F, m, r0, nr, SB * q, min(SB, k - SB * q));
       cp_async_commit();
+    }
+    if (!started) {  // the unit's factor blocks are on their way; its vectors are the predecessor's
+      wait_previous();
+      started = true;
     }
     T wrow[NR];
     if (fin && g == 0) {
@@ -1853,6 +1888,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
       else publish_add(fa.counters + u.cnt);
     }
   }
+  next_may_start();
   cp_async_wait_all();
 }
 
@@ -1875,6 +1911,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
   const int cl = g + 4 * ((lane >> 1) & 15);
   if (t == 0) s_tk[0] = atomicAdd(fa.ticket, 1);
   __syncthreads();
+  bool started = false;
   for (int par = 0;; par ^= 1) {
     const int tk = s_tk[par];
     if (tk >= fa.count) break;
@@ -1903,6 +1940,10 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
         cp_block(stage + j * SB * SB, F, m, r0, nr, c0, wc);
       }
       cp_async_commit();
+    }
+    if (!started) {  // the unit's factor blocks are on their way; its vectors are the predecessor's
+      wait_previous();
+      started = true;
     }
     T wrow[NR];
     if (fin && t < SB) {
@@ -2042,6 +2083,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
       else publish_add(fa.counters + u.cnt);
     }
   }
+  next_may_start();
   cp_async_wait_all();
 }
 
@@ -2109,6 +2151,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_mrhs(const double* __restrict__ 
   const int t = threadIdx.x, i = t & 63, g = t >> 6;
   if (t == 0) s_tk[0] = atomicAdd(fa.ticket, 1);
   __syncthreads();
+  bool started = false;
   for (int par = 0;; par ^= 1) {
     const int tk = s_tk[par];
     if (tk >= fa.count) break;
@@ -2132,6 +2175,10 @@ __global__ void __launch_bounds__(256, 2) k_fwd_mrhs(const double* __restrict__ 
     }
     // final pivot unit: its inverted diagonal block and its own rows of W do not
     // depend on this launch
+    if (!started) {
+      wait_previous();
+      started = true;
+    }
     double dpre[16], wrow[RPT];
     if (fin && piv) {
       const double* D = Dinv + u.dinv_off + (int64_t)R * SB * SB;
@@ -2257,6 +2304,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_mrhs(const double* __restrict__ 
       else publish_add(fa.counters + u.cnt);
     }
   }
+  next_may_start();
   cp_async_wait_all();
 }
 
@@ -2274,6 +2322,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_mrhs(const double* __restrict__ 
   const int t = threadIdx.x, c = t & 63, g = t >> 6;
   if (t == 0) s_tk[0] = atomicAdd(fa.ticket, 1);
   __syncthreads();
+  bool started = false;
   for (int par = 0;; par ^= 1) {
     const int tk = s_tk[par];
     if (tk >= fa.count) break;
@@ -2301,6 +2350,10 @@ __global__ void __launch_bounds__(256, 2) k_bwd_mrhs(const double* __restrict__ 
         cp_block_ls(Lst[j], F, m, rr0, nrr, c0, wc);
       }
       cp_async_commit();
+    }
+    if (!started) {
+      wait_previous();
+      started = true;
     }
     double dpre[16], wrow[RPT];
     if (fin) {
@@ -2427,6 +2480,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_mrhs(const double* __restrict__ 
       else publish_add(fa.counters + u.cnt);
     }
   }
+  next_may_start();
   cp_async_wait_all();
 }
 
@@ -2711,7 +2765,7 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
   };
   for (int l = 0; l < nlev; ++l) {
     const LevelPlan& lp = sy.levels[l];
-    k_fwd_gather<T><<<grid_of(lp.assemble.ctas), kSolveRows, 0, s>>>(W, b, a, kids, tasks + lp.assemble.off,
+    launch_next(k_fwd_gather<T>, grid_of(lp.assemble.ctas), kSolveRows, 0, s, W, b, a, kids, tasks + lp.assemble.off,
                                                                      prefix + lp.assemble.pre, lp.assemble.count);
     ++launches;
     if (lp.fwd_count == 0) continue;
@@ -2721,16 +2775,16 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
     f.ticket = tickets + 2 * l;
     f.flags = fflags;
     if constexpr (MR)
-      k_fwd_mrhs<RPT><<<grid(lp.fwd_count, 0), 256, ysm, s>>>(L, Dinv, W, part, a.nrhs, f);
+      launch_next(k_fwd_mrhs<RPT>, grid(lp.fwd_count, 0), 256, ysm, s, L, Dinv, W, part, a.nrhs, f);
     else if constexpr (STREAM)
-      k_fwd_stream<T, RPT><<<grid(lp.fwd_count, 0), 256, ysm, s>>>(L, Dinv, W, part, a.nrhs, f);
+      launch_next(k_fwd_stream<T, RPT>, grid(lp.fwd_count, 0), 256, ysm, s, L, Dinv, W, part, a.nrhs, f);
     else
-      k_fwd_level<T, RPT><<<grid(lp.fwd_count, 0), 256, ysm, s>>>(L, Dinv, W, part, a.nrhs, f);
+      launch_next(k_fwd_level<T, RPT>, grid(lp.fwd_count, 0), 256, ysm, s, L, Dinv, W, part, a.nrhs, f);
     ++launches;
   }
   for (int l = nlev - 1; l >= 0; --l) {
     const LevelPlan& lp = sy.levels[l];
-    k_bwd_init<T><<<grid_of(lp.assemble.ctas), kSolveRows, 0, s>>>(W, x, a, tasks + lp.assemble.off,
+    launch_next(k_bwd_init<T>, grid_of(lp.assemble.ctas), kSolveRows, 0, s, W, x, a, tasks + lp.assemble.off,
                                                                    prefix + lp.assemble.pre, lp.assemble.count);
     ++launches;
     if (lp.bwd_count == 0) continue;
@@ -2740,11 +2794,11 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
     f.ticket = tickets + 2 * l + 1;
     f.flags = bflags;
     if constexpr (MR)
-      k_bwd_mrhs<RPT><<<grid(lp.bwd_count, 1), 256, ysm, s>>>(L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
+      launch_next(k_bwd_mrhs<RPT>, grid(lp.bwd_count, 1), 256, ysm, s, L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
     else if constexpr (STREAM)
-      k_bwd_stream<T, RPT><<<grid(lp.bwd_count, 1), 256, ysm, s>>>(L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
+      launch_next(k_bwd_stream<T, RPT>, grid(lp.bwd_count, 1), 256, ysm, s, L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
     else
-      k_bwd_level<T, RPT><<<grid(lp.bwd_count, 1), 256, ysm, s>>>(L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
+      launch_next(k_bwd_level<T, RPT>, grid(lp.bwd_count, 1), 256, ysm, s, L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
     ++launches;
   }
 }
