@@ -767,16 +767,13 @@ std::string TransientSolve::refine(double* x) {
 void TransientSolve::eval_receivers(int t) {
   if (t < tlf_ || t > tll_) return;
   const int li = t - tlf_;
-  if (rop_b_.nrec) {
-    launch_receivers(d_rb_ptr_, d_rb_col_, d_rb_val_, d_rb_src_, 3 * rop_b_.nrec, layer(t), n_,
-                     d_vb_ + (size_t)li * 3 * rop_b_.nrec, s_);
-    ++launches_;
-  }
-  if (rop_e_.nrec) {
-    launch_receivers(d_re_ptr_, d_re_col_, d_re_val_, d_re_src_, 3 * rop_e_.nrec, layer(t), n_,
-                     d_ve_ + (size_t)li * 3 * rop_e_.nrec, s_);
-    ++launches_;
-  }
+  const ReceiverRows b{d_rb_ptr_, d_rb_col_, d_rb_val_, d_rb_src_, 3 * rop_b_.nrec,
+                       d_vb_ + (size_t)li * 3 * rop_b_.nrec};
+  const ReceiverRows e{d_re_ptr_, d_re_col_, d_re_val_, d_re_src_, 3 * rop_e_.nrec,
+                       d_ve_ + (size_t)li * 3 * rop_e_.nrec};
+  if (b.nrows + e.nrows == 0) return;
+  launch_receivers(b, e, layer(t), n_, s_);
+  ++launches_;
 }
 
 std::string TransientSolve::run() {

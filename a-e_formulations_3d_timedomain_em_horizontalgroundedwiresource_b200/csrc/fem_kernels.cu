@@ -234,18 +234,26 @@ __global__ void __launch_bounds__(256) k_history_rhs_multi(const int64_t* __rest
   }
 }
 
-__global__ void k_receivers(const int64_t* __restrict__ rowptr, const int* __restrict__ col,
-                            const double* __restrict__ val, const int* __restrict__ src, int nrows,
-                            const double* __restrict__ u, int64_t ld, double* __restrict__ out) {
-  const int row = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= nrows) return;
-  const double* x = u + (int64_t)src[row] * ld;
+// One CTA per operator row, the B rows first and then the E rows: a row (one component of
+// one receiver) holds the smoothing subdomain's edges, several hundred to a few thousand,
+// and with a warp each the two launches were 42 us a step at 40^3; the one is 16.
+__global__ void __launch_bounds__(128) k_receivers(ReceiverRows b, ReceiverRows e, const double* __restrict__ u,
+                                                   int64_t ld) {
+  __shared__ double red[4];
+  const bool first = (int)blockIdx.x < b.nrows;
+  const int64_t* rowptr = first ? b.rowptr : e.rowptr;
+  const int* col = first ? b.col : e.col;
+  const double* val = first ? b.val : e.val;
+  const int row = first ? blockIdx.x : blockIdx.x - b.nrows;
+  const double* x = u + (int64_t)(first ? b.src : e.src)[row] * ld;
   double acc = 0.0;
-  for (int64_t q = rowptr[row] + lane; q < rowptr[row + 1]; q += 32) acc = fma(val[q], x[col[q]], acc);
+  const int64_t end = rowptr[row + 1];
+  for (int64_t q = rowptr[row] + threadIdx.x; q < end; q += 128) acc = fma(__ldg(val + q), x[__ldg(col + q)], acc);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if (lane == 0) out[row] = acc;
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) (first ? b.out : e.out)[row] = (red[0] + red[1]) + (red[2] + red[3]);
 }
 
 __global__ void k_time_diff(const double* __restrict__ F, int nt, int nser, int t0,
@@ -494,11 +502,9 @@ void launch_anomaly_rhs(const int64_t* rowptr, const int* col, const double* Cds
   k_anomaly_rhs<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(rowptr, col, Cds, En, bound, n, npls, rhs);
 }
 
-void launch_receivers(const int64_t* rowptr, const int* col, const double* val, const int* src,
-                      int nrows, const double* u, int64_t ld, double* out, cudaStream_t s) {
-  if (nrows <= 0) return;
-  const int64_t threads = (int64_t)nrows * 32;
-  k_receivers<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(rowptr, col, val, src, nrows, u, ld, out);
+void launch_receivers(const ReceiverRows& b, const ReceiverRows& e, const double* u, int64_t ld, cudaStream_t s) {
+  const int rows = b.nrows + e.nrows;
+  if (rows > 0) k_receivers<<<(unsigned)rows, 128, 0, s>>>(b, e, u, ld);
 }
 
 void launch_time_diff(const double* series, int nt, int nser, int t0, const double* time,

@@ -36,7 +36,16 @@ void launch_history_rhs(const int64_t* rowptr, const int* col, const double* Cva
                         const double* u2, double m1, double m2, const double* S, double coef,
                         const uint8_t* bound, int n, int npls, double* rhs, double* scratch, cudaStream_t s);
 
-// Receiver values: out[row] = sum_j R[row, j] * u[j, src[row]] for every operator row.
+// Rows of a receiver operator (CSR over edges, src: the source a row belongs to).
+struct ReceiverRows {
+  const int64_t* rowptr;
+  const int* col;
+  const double* val;
+  const int* src;
+  int nrows;
+  double* out;
+};
+
 // Primary-secondary source of one time layer.  The normal field f (float, V/m,
 // nanom values per source, source-major) of the anomalous edges idx becomes edge
 // degrees of freedom En = f * len * 0.5 (the other entries of En stay as they are,
@@ -46,8 +55,8 @@ void launch_normal_field(const float* f, const int* idx, const double* len, int 
 void launch_anomaly_rhs(const int64_t* rowptr, const int* col, const double* Cds, const double* En,
                         const uint8_t* bound, int n, int npls, double* rhs, cudaStream_t s);
 
-void launch_receivers(const int64_t* rowptr, const int* col, const double* val, const int* src,
-                      int nrows, const double* u, int64_t ld, double* out, cudaStream_t s);
+// Receiver values: out[row] = sum_j R[row, j] * u[j, src[row]] for every row of both operators.
+void launch_receivers(const ReceiverRows& b, const ReceiverRows& e, const double* u, int64_t ld, cudaStream_t s);
 
 // A = mult * C + B on every entry of the full CSR, with the diagonal scaled by
 // (1 + 1e-12); rows and columns of Dirichlet edges are left out (their values
