@@ -57,9 +57,9 @@ __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.w
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... P, class... A>
-void launch_next(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
+void launch_next(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
@@ -871,6 +871,8 @@ struct SolveArgs {
   int64_t ld;
 };
 
+constexpr int kColChunk = 8;  // right-hand sides per CTA of the front-vector kernels (grid.y chunks)
+
 // Front vectors of a level: the right-hand side on the pivot rows plus what the children
 // left on the front's rows, gathered in child order (one launch where setting up and
 // adding one child after another was three).
@@ -888,7 +890,7 @@ __global__ void k_fwd_gather(T* W, const double* __restrict__ b, SolveArgs a, Ki
   T* w = W + a.w_off[s] * a.nrhs;
   const int pos = (i < k) ? a.rows[a.rows_off[s] + i] : -1;
   const int q0 = kids.ptr[s], q1 = kids.ptr[s + 1];
-  for (int r0 = 0; r0 < a.nrhs; r0 += N) {
+  for (int r0 = kColChunk * blockIdx.y; r0 < min(a.nrhs, kColChunk * ((int)blockIdx.y + 1)); r0 += N) {
     T v[N];
 #pragma unroll
     for (int e = 0; e < N; ++e) v[e] = (i < k && r0 + e < a.nrhs) ? (T)b[pos + (r0 + e) * a.ld] : (T)0;
@@ -983,7 +985,9 @@ __global__ void k_bwd_init(T* __restrict__ W, const double* __restrict__ x, Solv
   if (i < k || i >= m) return;
   T* w = W + a.w_off[s] * a.nrhs;
   const int pos = a.rows[a.rows_off[s] + i];
-  for (int r = 0; r < a.nrhs; ++r) w[i + (int64_t)r * m] = (T)x[pos + r * a.ld];
+#pragma unroll 4
+  for (int r = kColChunk * blockIdx.y; r < min(a.nrhs, kColChunk * ((int)blockIdx.y + 1)); ++r)
+    w[i + (int64_t)r * m] = (T)x[pos + r * a.ld];
 }
 
 // Partial sums of L[j1:m, panel]^T W[j1:m] over one row chunk.
@@ -1138,6 +1142,10 @@ struct FusedArgs {
   int* flags;              // one per pivot block (zeroed before the solve)
   int* counters;           // finished chunk units per row (zeroed before the solve)
   int* err;                // set to 1 when a wait gave up (the solver's err[1])
+  // many-column kernels: columns per group; group blockIdx.y has its own tickets, flags and
+  // counters, `stride` ints after those of the group before
+  int cols = 0;
+  int64_t stride = 0;
 };
 
 // A level-solve unit as unpacked from its 64-byte record.
@@ -1182,7 +1190,7 @@ __device__ __forceinline__ void publish_partial(T* part, const T (&acc)[RPT], in
 // when the row has no chunk units).
 template <class T, int RPT>
 __device__ __forceinline__ void gather_partials(const T* part, int nparts, int nr_rhs, const int* counter, int* err,
-                                                T (&acc)[RPT]) {
+                                                T (&acc)[RPT], int nr_all) {
   if (nparts == 0) return;
   if (threadIdx.x == 0) wait_count(counter, nparts, err);
   __syncthreads();
@@ -1192,7 +1200,7 @@ __device__ __forceinline__ void gather_partials(const T* part, int nparts, int n
     const int r = g + 4 * j;
     if (r >= nr_rhs) continue;
     T tot = __ldcg(part + i + SB * r);
-    for (int c = 1; c < nparts; ++c) tot += __ldcg(part + (int64_t)c * SB * nr_rhs + i + SB * r);
+    for (int c = 1; c < nparts; ++c) tot += __ldcg(part + (int64_t)c * SB * nr_all + i + SB * r);
     acc[j] = tot;
   }
 }
@@ -1352,7 +1360,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_level(const T* __restrict__ L, c
 #pragma unroll
   for (int j = 0; j < RPT; ++j) tot[j] = (T)0;
   // the chunk partials of this row are ready long before the last block's flag
-  if (fin) gather_partials<T, RPT>(my_part, u.nparts, nr_rhs, fa.counters + u.cnt, fa.err, tot);
+  if (fin) gather_partials<T, RPT>(my_part, u.nparts, nr_rhs, fa.counters + u.cnt, fa.err, tot, nr_rhs);
   T pre[16];
   if (lo < hi) load_block(pre, F, m, r0, nr, SB * lo, min(SB, k - SB * lo));
   for (int q = lo; q < hi; ++q) {
@@ -1507,7 +1515,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_level(const T* __restrict__ L, c
   T tot[RPT];
 #pragma unroll
   for (int j = 0; j < RPT; ++j) tot[j] = (T)0;
-  if (fin) gather_partials<T, RPT>(my_part, u.nparts, nr_rhs, fa.counters + u.cnt, fa.err, tot);
+  if (fin) gather_partials<T, RPT>(my_part, u.nparts, nr_rhs, fa.counters + u.cnt, fa.err, tot, nr_rhs);
   auto rows_of = [&](int R, int& r0, int& nr) {
     r0 = (R < pb) ? SB * R : k + SB * (R - pb);
     nr = min(SB, (R < pb ? k : m) - r0);
@@ -2141,11 +2149,16 @@ __device__ __forceinline__ void ld_vec_block(double* Vs, int ysl, const double* 
 
 template <int RPT>
 __global__ void __launch_bounds__(256, 2) k_fwd_mrhs(const double* __restrict__ L, const double* __restrict__ Dinv,
-                                                  double* W, double* part, int nr_rhs, FusedArgs fa) {
+                                                  double* W, double* part, int nr_all, FusedArgs fa) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   double(*Lst)[SB][kLdL] = reinterpret_cast<double(*)[SB][kLdL]>(sm_raw);
   double* Yst = reinterpret_cast<double*>(sm_raw + sizeof(double) * kMrStages * SB * kLdL);
   __shared__ int s_tk[2], s_ready;
+  // this group's columns [first, first + nr_rhs) of nr_all
+  const int first = fa.cols * (int)blockIdx.y, nr_rhs = min(fa.cols, nr_all - first);
+  fa.ticket += fa.stride * blockIdx.y;
+  fa.flags += fa.stride * blockIdx.y;
+  fa.counters += fa.stride * blockIdx.y;
   constexpr int NTW = (RPT + 3) / 4;
   const int ysl = ys_ld(nr_rhs), ntl = (nr_rhs + 7) / 8;
   const int t = threadIdx.x, i = t & 63, g = t >> 6;
@@ -2165,7 +2178,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_mrhs(const double* __restrict__ 
     const int r0 = piv ? SB * R : k + SB * (R - pb);
     const int nr = min(SB, (piv ? k : m) - r0);
     const double* F = L + u.l_off;
-    double* w = W + u.w_off * nr_rhs;
+    double* w = W + u.w_off * nr_all + (int64_t)first * m;
     const int* flags = fa.flags + u.flag0;
 #pragma unroll
     for (int j = 0; j < kMrStages; ++j) {
@@ -2193,11 +2206,11 @@ __global__ void __launch_bounds__(256, 2) k_fwd_mrhs(const double* __restrict__ 
         wrow[j] = (r < nr_rhs && i < nr) ? __ldcg(w + r0 + i + (int64_t)r * m) : 0.0;
       }
     }
-    double* my_part = part + (int64_t)u.slot * SB * nr_rhs;
+    double* my_part = part + (int64_t)u.slot * SB * nr_all + SB * first;
     double tot[RPT];
 #pragma unroll
     for (int j = 0; j < RPT; ++j) tot[j] = 0.0;
-    if (fin) gather_partials<double, RPT>(my_part, u.nparts, nr_rhs, fa.counters + u.cnt, fa.err, tot);
+    if (fin) gather_partials<double, RPT>(my_part, u.nparts, nr_rhs, fa.counters + u.cnt, fa.err, tot, nr_all);
     // flags of a front are set in chain order: the newest flag of the range stands
     // for all of them (see k_fwd_stream)
     const bool chain = fin && piv;
@@ -2311,12 +2324,17 @@ __global__ void __launch_bounds__(256, 2) k_fwd_mrhs(const double* __restrict__ 
 template <int RPT>
 __global__ void __launch_bounds__(256, 2) k_bwd_mrhs(const double* __restrict__ L, const double* __restrict__ Dinv,
                                                   double* W, double* part, double* __restrict__ x,
-                                                  const int* __restrict__ rows, int64_t ldx, int nr_rhs,
+                                                  const int* __restrict__ rows, int64_t ldx, int nr_all,
                                                   FusedArgs fa) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   double(*Lst)[SB][kLdL] = reinterpret_cast<double(*)[SB][kLdL]>(sm_raw);
   double* Wst = reinterpret_cast<double*>(sm_raw + sizeof(double) * kMrStages * SB * kLdL);
   __shared__ int s_tk[2], s_ready;
+  // this group's columns [first, first + nr_rhs) of nr_all
+  const int first = fa.cols * (int)blockIdx.y, nr_rhs = min(fa.cols, nr_all - first);
+  fa.ticket += fa.stride * blockIdx.y;
+  fa.flags += fa.stride * blockIdx.y;
+  fa.counters += fa.stride * blockIdx.y;
   constexpr int NTW = (RPT + 3) / 4;
   const int ysl = ys_ld(nr_rhs), ntl = (nr_rhs + 7) / 8;
   const int t = threadIdx.x, c = t & 63, g = t >> 6;
@@ -2334,7 +2352,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_mrhs(const double* __restrict__ 
     const int pb = (k + SB - 1) / SB;
     const int c0 = SB * p, wc = min(SB, k - c0);
     const double* F = L + u.l_off;
-    double* w = W + u.w_off * nr_rhs;
+    double* w = W + u.w_off * nr_all + (int64_t)first * m;
     const int* flags = fa.flags + u.flag0;
     auto rows_of = [&](int Rr, int& rr0, int& nrr) {
       rr0 = (Rr < pb) ? SB * Rr : k + SB * (Rr - pb);
@@ -2369,11 +2387,11 @@ __global__ void __launch_bounds__(256, 2) k_bwd_mrhs(const double* __restrict__ 
         wrow[j] = (r < nr_rhs && c < wc) ? __ldcg(w + c0 + c + (int64_t)r * m) : 0.0;
       }
     }
-    double* my_part = part + (int64_t)u.slot * SB * nr_rhs;
+    double* my_part = part + (int64_t)u.slot * SB * nr_all + SB * first;
     double tot[RPT];
 #pragma unroll
     for (int j = 0; j < RPT; ++j) tot[j] = 0.0;
-    if (fin) gather_partials<double, RPT>(my_part, u.nparts, nr_rhs, fa.counters + u.cnt, fa.err, tot);
+    if (fin) gather_partials<double, RPT>(my_part, u.nparts, nr_rhs, fa.counters + u.cnt, fa.err, tot, nr_all);
     // flags are set last column first: flag lo stands for every pivot row block of
     // the range (see k_bwd_stream); update rows need no flag
     if (t == 0) {
@@ -2469,7 +2487,7 @@ __global__ void __launch_bounds__(256, 2) k_bwd_mrhs(const double* __restrict__ 
       for_acc<NTW>(xv, ntl, [&](int row, int r, double v) {
         if (row < wc && r < nr_rhs) {
           w[c0 + row + (int64_t)r * m] = v;
-          x[rows[u.w_off + c0 + row] + (int64_t)r * ldx] = v;
+          x[rows[u.w_off + c0 + row] + (int64_t)(first + r) * ldx] = v;
         }
       });
     }
@@ -2533,6 +2551,8 @@ __global__ void __launch_bounds__(256) k_diag_inverse(const T* __restrict__ L, T
   } while (0)
 
 inline unsigned grid_of(int64_t ctas) { return (unsigned)ctas; }
+// front-vector kernels: row blocks of the fronts x chunks of right-hand sides
+inline dim3 front_grid(int64_t ctas, int nrhs) { return dim3((unsigned)ctas, (unsigned)((nrhs + kColChunk - 1) / kColChunk)); }
 // dst[i] = (float)src[i], two elements per thread and iteration (16-byte loads
 // where the pair is aligned; n may be odd), grid-stride.
 __global__ void __launch_bounds__(256) k_round_to_float(const double* __restrict__ src, float* __restrict__ dst,
@@ -2706,7 +2726,7 @@ int launch_solve(const Symbolic& sy, const T* L, T* W, T* part, const double* b,
   int launches = 0;
   const size_t ysm = sizeof(T) * P * a.nrhs;
   for (const LevelPlan& lp : sy.levels) {
-    k_fwd_gather<T><<<grid_of(lp.assemble.ctas), kSolveRows, 0, s>>>(W, b, a, kids, tasks + lp.assemble.off,
+    k_fwd_gather<T><<<front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s>>>(W, b, a, kids, tasks + lp.assemble.off,
                                                                      prefix + lp.assemble.pre, lp.assemble.count);
     ++launches;
     for (const PanelStep& ps : lp.panels) {
@@ -2721,7 +2741,7 @@ int launch_solve(const Symbolic& sy, const T* L, T* W, T* part, const double* b,
   }
   for (int l = (int)sy.levels.size() - 1; l >= 0; --l) {
     const LevelPlan& lp = sy.levels[l];
-    k_bwd_init<T><<<grid_of(lp.assemble.ctas), kSolveRows, 0, s>>>(W, x, a, tasks + lp.assemble.off,
+    k_bwd_init<T><<<front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s>>>(W, x, a, tasks + lp.assemble.off,
                                                                    prefix + lp.assemble.pre, lp.assemble.count);
     ++launches;
     for (int p = (int)lp.panels.size() - 1; p >= 0; --p) {
@@ -2742,6 +2762,29 @@ int launch_solve(const Symbolic& sy, const T* L, T* W, T* part, const double* b,
   return launches;
 }
 
+// ints of one group's tickets, flags and counters
+inline int64_t sync_ints(const Symbolic& sy) {
+  return 2 * (int64_t)sy.levels.size() + 2 * sy.n_flags + sy.n_counters;
+}
+// Column groups of the many-column solves: groups of at least 8 columns, at most four.
+inline int max_col_groups(int nrhs) { return nrhs > 16 ? 4 : (nrhs > 8 ? 2 : 1); }
+// A level's groups run side by side, each with a chain of its own over fewer columns: a
+// link is about 3.2 us and 0.17 us a column.  Each group reads the level's factor, about
+// 4 TB/s: the fewest groups that leave the slower of the two least.
+inline int col_groups(const LevelPlan& lp, int nrhs) {
+  int best = 1;
+  double least = 0;
+  for (int g = 1; g <= max_col_groups(nrhs); g *= 2) {
+    const double cols = (nrhs + g - 1) / g;
+    const double us = std::max((double)lp.chain * (3.2 + 0.17 * cols), g * 8.0 * (double)lp.entries / 4e6);
+    if (g == 1 || us < 0.95 * least) {
+      least = us;
+      best = g;
+    }
+  }
+  return best;
+}
+
 // One forward and one backward launch per level (plus the front-vector set-up).
 // STREAM: the persistent streaming kernels (nrhs <= NR <= 4, grid = resident
 // CTAs); MR: the persistent many-column kernels (FP64, 3..32 columns, grid =
@@ -2758,14 +2801,15 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
   int* fflags = sync + 2 * nlev;
   int* bflags = fflags + sy.n_flags;
   fa.counters = bflags + sy.n_flags;
-  cudaMemsetAsync(sync, 0, sizeof(int) * (2 * nlev + 2 * sy.n_flags + sy.n_counters), s);
+  fa.stride = sync_ints(sy);
+  cudaMemsetAsync(sync, 0, sizeof(int) * (size_t)(fa.stride * (MR ? max_col_groups(a.nrhs) : 1)), s);
   const size_t ysm = STREAM ? stream_smem<T>() : (MR ? mr_smem() : sizeof(T) * SB * ys_ld(a.nrhs));
   auto grid = [&](int64_t count, int dir) {
     return (STREAM || MR) ? (unsigned)std::min<int64_t>(count, resident[dir]) : grid_of(count);
   };
   for (int l = 0; l < nlev; ++l) {
     const LevelPlan& lp = sy.levels[l];
-    launch_next(k_fwd_gather<T>, grid_of(lp.assemble.ctas), kSolveRows, 0, s, W, b, a, kids, tasks + lp.assemble.off,
+    launch_next(k_fwd_gather<T>, front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s, W, b, a, kids, tasks + lp.assemble.off,
                                                                      prefix + lp.assemble.pre, lp.assemble.count);
     ++launches;
     if (lp.fwd_count == 0) continue;
@@ -2774,8 +2818,16 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
     f.count = lp.fwd_count;
     f.ticket = tickets + 2 * l;
     f.flags = fflags;
-    if constexpr (MR)
-      launch_next(k_fwd_mrhs<RPT>, grid(lp.fwd_count, 0), 256, ysm, s, L, Dinv, W, part, a.nrhs, f);
+    if constexpr (MR) {
+      const int groups = col_groups(lp, a.nrhs);
+      f.cols = (a.nrhs + groups - 1) / groups;
+      auto go = [&](auto kernel) {
+        launch_next(kernel, dim3((unsigned)std::min<int64_t>(lp.fwd_count, std::max(1, resident[0] / groups)),
+                                 (unsigned)groups), 256, ysm, s, L, Dinv, W, part, a.nrhs, f);
+      };
+      f.cols <= 4 ? go(k_fwd_mrhs<1>) : f.cols <= 8 ? go(k_fwd_mrhs<2>) : f.cols <= 16 ? go(k_fwd_mrhs<4>)
+                                                                                     : go(k_fwd_mrhs<8>);
+    }
     else if constexpr (STREAM)
       launch_next(k_fwd_stream<T, RPT>, grid(lp.fwd_count, 0), 256, ysm, s, L, Dinv, W, part, a.nrhs, f);
     else
@@ -2784,7 +2836,7 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
   }
   for (int l = nlev - 1; l >= 0; --l) {
     const LevelPlan& lp = sy.levels[l];
-    launch_next(k_bwd_init<T>, grid_of(lp.assemble.ctas), kSolveRows, 0, s, W, x, a, tasks + lp.assemble.off,
+    launch_next(k_bwd_init<T>, front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s, W, x, a, tasks + lp.assemble.off,
                                                                    prefix + lp.assemble.pre, lp.assemble.count);
     ++launches;
     if (lp.bwd_count == 0) continue;
@@ -2793,8 +2845,16 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
     f.count = lp.bwd_count;
     f.ticket = tickets + 2 * l + 1;
     f.flags = bflags;
-    if constexpr (MR)
-      launch_next(k_bwd_mrhs<RPT>, grid(lp.bwd_count, 1), 256, ysm, s, L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
+    if constexpr (MR) {
+      const int groups = col_groups(lp, a.nrhs);
+      f.cols = (a.nrhs + groups - 1) / groups;
+      auto go = [&](auto kernel) {
+        launch_next(kernel, dim3((unsigned)std::min<int64_t>(lp.bwd_count, std::max(1, resident[1] / groups)),
+                                 (unsigned)groups), 256, ysm, s, L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
+      };
+      f.cols <= 4 ? go(k_bwd_mrhs<1>) : f.cols <= 8 ? go(k_bwd_mrhs<2>) : f.cols <= 16 ? go(k_bwd_mrhs<4>)
+                                                                                     : go(k_bwd_mrhs<8>);
+    }
     else if constexpr (STREAM)
       launch_next(k_bwd_stream<T, RPT>, grid(lp.bwd_count, 1), 256, ysm, s, L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
     else
@@ -2834,18 +2894,8 @@ int launch_solve_mr(const Symbolic& sy, const double* L, const double* Dinv, dou
                     double* x, SolveArgs a, const Kids& kids, const int* tasks, const int64_t* prefix, FusedArgs fa, int* sync, const int (&resident)[2],
                     cudaStream_t s) {
   int launches = 0;
-#define TDEM_MR(R) \
-  launch_level_solves<double, R, false, true>(sy, L, Dinv, W, part, b, x, a, kids, tasks, prefix, \
-                                              fa, sync, resident, launches, s)
-  if (a.nrhs <= 4)
-    TDEM_MR(1);
-  else if (a.nrhs <= 8)
-    TDEM_MR(2);
-  else if (a.nrhs <= 16)
-    TDEM_MR(4);
-  else
-    TDEM_MR(8);
-#undef TDEM_MR
+  launch_level_solves<double, 8, false, true>(sy, L, Dinv, W, part, b, x, a, kids, tasks, prefix, fa, sync, resident,
+                                              launches, s);
   return launches;
 }
 
@@ -2962,7 +3012,7 @@ int64_t GpuCholesky::bytes_needed(const Symbolic& sy, int nrhs_max, int precisio
                      sy.rel_off.size() + sy.rows_off.size() + sy.task_prefix.size() + sy.dinv_off.size());
   b += 4 * (int64_t)(sy.front_m.size() + sy.front_k.size() + sy.rel.size() + sy.rows_all.size() + sy.tasks.size() +
                      sy.front_parent.size() + sy.front_c0.size() + sy.solve_items.size() + sy.solve_units.size() +
-                     2 * sy.levels.size() + 2 * sy.n_flags + sy.n_counters + 4);
+                     max_col_groups((int)nr) * sync_ints(sy) + 4);
   return b;
 }
 
@@ -3016,8 +3066,7 @@ std::string GpuCholesky::setup(Symbolic&& sy, const std::vector<int>& perm_to_ve
   if (!(e = upload(&d_dinv_off_, sy_.dinv_off, s)).empty()) return e;
   if (!(e = upload(&d_units_, sy_.solve_units, s)).empty()) return e;
   if (!(e = alloc(&d_spart_, elem_ * std::max<int64_t>(1, sy_.solve_slots) * kPanel * nrhs_max_)).empty()) return e;
-  if (!(e = alloc((void**)&d_sync_,
-                  sizeof(int) * (2 * sy_.levels.size() + 2 * sy_.n_flags + sy_.n_counters + 1))).empty())
+  if (!(e = alloc((void**)&d_sync_, sizeof(int) * (size_t)(max_col_groups(nrhs_max_) * sync_ints(sy_) + 1))).empty())
     return e;
   if (!(e = alloc((void**)&d_err_, 3 * sizeof(int))).empty()) return e;
   TDEM_CUDA_TRY(cudaMemsetAsync(d_err_, 0, 3 * sizeof(int), s));

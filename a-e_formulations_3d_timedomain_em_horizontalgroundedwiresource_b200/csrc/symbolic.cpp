@@ -664,6 +664,10 @@ std::string analyse(int n, const int64_t* rowptr, const int* colind, const doubl
       }
       add_tasks(sy, lp.assemble, lp.fronts, ct);
       add_tasks(sy, lp.assemble_cols, lp.fronts, cc);
+      for (int s : lp.fronts) {
+        lp.chain = std::max(lp.chain, (int)cdiv(sy.front_k[s], kPanel));
+        lp.entries += (int64_t)sy.front_m[s] * sy.front_k[s];
+      }
     }
     int kmax = 0;
     for (int s : lp.fronts) kmax = std::max(kmax, sy.front_k[s]);

@@ -109,6 +109,8 @@ struct LevelPlan {
   // waits for has a smaller ticket.
   int64_t fwd_off = 0, fwd_count = 0;
   int64_t bwd_off = 0, bwd_count = 0;
+  int chain = 0;        // pivot blocks of the level's longest front (links of its chain)
+  int64_t entries = 0;  // factor entries of the level
 };
 
 struct Symbolic {
