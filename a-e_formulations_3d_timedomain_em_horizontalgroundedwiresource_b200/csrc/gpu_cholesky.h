@@ -198,6 +198,7 @@ class GpuCholesky {
   int64_t* d_dinv_off_ = nullptr;
   void* d_dinv_[kMaxSlots] = {};  // inverted diagonal blocks per slot
   int* d_sync_ = nullptr;        // level tickets + pivot-block flags + row counters of one solve
+  void* d_mail_ = nullptr;       // solved values of the streaming solves' chains (FusedArgs::mail)
   int* d_units_ = nullptr;       // level-solve units
   void* d_spart_ = nullptr;      // level-solve partial sums (slots x 64 x nrhs)
   std::vector<void*> allocs_;
