@@ -1662,20 +1662,22 @@ __global__ void __launch_bounds__(256, 2) k_bwd_level(const T* __restrict__ L, c
 // Streaming level solves for one or two right-hand sides.
 //
 // Persistent CTAs (as many as fit on the device) take units by ticket until the
-// level's list is exhausted; the next ticket is taken when a unit starts, so its
-// latency hides behind the unit's work.  Each thread copies its own elements of
-// the unit's blocks into shared memory with cp.async, kStages blocks ahead of
-// their use (and the inverted diagonal block of a final unit at the start), so
-// a CTA keeps several 32 KB loads in flight without holding them in registers;
-// since a thread only reads back what it copied, no CTA barrier is needed
-// between copy and use.  A link of the dependency chain waits for each pivot block in
-// two of its warps, which bring the block's values into shared memory for the others:
-// with every warp polling for itself the last one saw a flag up to 4 us after it was
-// set, and each link of a 3,264-pivot front took 6.3 us forward and 2.5 backward where it now
-// takes 1.9 and 2.3.  The four column groups (forward) or 64 rows (backward) of a
-// block are combined once per unit, in a fixed order, so results are deterministic.
+// level's list is exhausted; the next ticket is taken when a unit starts.  Each thread
+// copies its own elements of the units' blocks into a ring of kStages shared-memory
+// buffers with cp.async (an inverted diagonal block is the last block of a final unit),
+// and the copies go on into the next unit while this one is summed; since a thread only
+// reads back what it copied, no CTA barrier is needed between copy and use.
+//
+// Solved values are read from the mailbox: one look by every thread for the whole unit,
+// and where some are still missing a link of the dependency chain takes its blocks one by
+// one (two warps wait and bring the values into shared memory for the others) and any
+// other unit waits for all of them.  A link takes 1.45 us forward and 1.6 backward (6.3 and
+// 2.5 with a flag that every warp polls for itself).  Reading ahead and the single look in
+// place of a flag and a read took the 40^3-cell step's solve from 1.31 to 1.24 ms.  The four
+// column groups (forward) or 64 rows (backward) of a block are combined once per unit, in a
+// fixed order, so results are deterministic.
 // ---------------------------------------------------------------------------
-constexpr int kStages = 2;
+constexpr int kStages = 3;
 
 // This thread's 16 elements (row t % 64, columns t / 64 + 4 e) of the 64 x 64
 // block at rows [r0, r0 + nr), columns [c0, c0 + nc) of F (zero outside) into
@@ -1742,11 +1744,46 @@ __device__ void wait_flag_backoff(const int* flag, int* err, unsigned sleep_max)
   atomicExch(err, 1);
 }
 
-
-// Dynamic shared memory of the streaming kernels: kStages block buffers and the
-// inverted diagonal block, 64 x 64 entries each.
+// The same for a value of the mailbox.
 template <class T>
-constexpr size_t stream_smem() { return sizeof(T) * (kStages + 1) * SB * SB; }
+__device__ void wait_mail_backoff(const T* p, int* err, unsigned sleep_max) {
+  unsigned ns = 32;
+  for (unsigned it = 0; it < kSpinLimit; ++it) {
+    if (!empty_mail(read_mail(p)) || ((it & 15) == 15 && *(volatile int*)err != 0)) return;
+    __nanosleep(ns);
+    ns = min(2 * ns, sleep_max);
+  }
+  atomicExch(err, 1);
+}
+
+// Loads per thread that cover the solved values of a unit's blocks.
+template <int NR>
+constexpr int kStageLoads = (kUnitBlocks * SB * NR + 255) / 256;
+
+// Dynamic shared memory of the streaming kernels: a ring of kStages block buffers.
+template <class T>
+constexpr size_t stream_smem() { return sizeof(T) * kStages * SB * SB; }
+
+// Place in the ring of block buffers: `depth` copies are under way or landed, the
+// oldest of them in slot `take`.  Every copy is one cp.async group of each thread.
+struct Ring {
+  int depth = 0, take = 0;
+  __device__ __forceinline__ int free_slot() const {
+    const int j = take + depth;
+    return j >= kStages ? j - kStages : j;
+  }
+  // waits for the calling thread's part of the oldest copy
+  __device__ __forceinline__ void wait_oldest() const {
+    static_assert(kStages == 3, "one case per possible depth");
+    if (depth >= 3) cp_async_wait<2>();
+    else if (depth == 2) cp_async_wait<1>();
+    else cp_async_wait<0>();
+  }
+  __device__ __forceinline__ void pop() {
+    take = take == kStages - 1 ? 0 : take + 1;
+    --depth;
+  }
+};
 
 // Forward unit, streaming form (see k_fwd_level for the unit's meaning).
 // Thread t holds row i = t % 64 of columns g + 4 e (g = t / 64, e < 16) of each
@@ -1756,15 +1793,45 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
                                                     T* part, int nr_rhs, FusedArgs fa) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   T* stage = reinterpret_cast<T*>(sm_raw);     // kStages x 4096
-  T* dsm = stage + kStages * SB * SB;          // inverted diagonal block, 4096
   __shared__ T red[4][SB][NR];  // per column group: partial row sums
   __shared__ T zs[SB][NR];      // pivot rows: w - sum, the input of the inverse
   __shared__ T ys[kUnitBlocks][SB][NR];  // y of every block of the unit (when staged)
-  __shared__ int s_tk[2], s_ready;
+  __shared__ int s_tk[2];
   const int t = threadIdx.x, i = t & 63, g = t >> 6, lane = t & 31;
   if (t == 0) s_tk[0] = atomicAdd(fa.ticket, 1);
   __syncthreads();
-  bool started = false;
+  // The copies run ahead of the sums: blocks [cq, chi) of the unit they have reached,
+  // then its inverted diagonal block cD (final pivot units), then the unit of ticket
+  // `ahead` (fa.count or more: none is known yet).
+  Ring ring;
+  int ahead = s_tk[0], cq = 0, chi = 0, cm = 0, ck = 0, cr0 = 0, cnr = 0;
+  const T *cF = L, *cD = nullptr;
+  auto top_up = [&]() {
+    while (ring.depth < kStages) {
+      if (cq >= chi && cD == nullptr) {
+        if (ahead >= fa.count) break;
+        const Unit v = load_unit(fa.units, ahead);
+        ahead = INT_MAX;
+        const int vpb = (v.k + SB - 1) / SB;
+        const bool vpiv = v.R < vpb;
+        cr0 = vpiv ? SB * v.R : v.k + SB * (v.R - vpb);
+        cnr = min(SB, (vpiv ? v.k : v.m) - cr0);
+        cq = v.lo, chi = v.hi, cm = v.m, ck = v.k;
+        cF = L + v.l_off;
+        if (v.fin != 0 && vpiv) cD = Dinv + v.dinv_off + (int64_t)v.R * SB * SB;
+        if (cq >= chi && cD == nullptr) break;  // a row of a front without pivots: nothing to read
+      }
+      const bool blk = cq < chi;
+      cp_block(stage + ring.free_slot() * SB * SB, blk ? cF : cD, blk ? cm : cnr, blk ? cr0 : 0, cnr, blk ? SB * cq : 0,
+               blk ? min(SB, ck - SB * cq) : cnr);
+      cp_async_commit();
+      ++ring.depth;
+      if (blk) ++cq;
+      else cD = nullptr;
+    }
+  };
+  top_up();
+  wait_previous();  // the first blocks are on their way; the vectors are the predecessor's
   for (int par = 0;; par ^= 1) {
     const int tk = s_tk[par];
     if (tk >= fa.count) break;
@@ -1777,22 +1844,8 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
     const bool piv = R < pb;
     const int r0 = piv ? SB * R : k + SB * (R - pb);
     const int nr = min(SB, (piv ? k : m) - r0);
-    const T* F = L + u.l_off;
     T* w = W + u.w_off * nr_rhs;
-    const int* flags = fa.flags + u.flag0;
     T* mail = static_cast<T*>(fa.mail) + (int64_t)u.flag0 * SB * NR;
-    // final pivot unit: the inverted diagonal block (independent of this launch)
-    if (fin && piv) cp_block(dsm, Dinv + u.dinv_off + (int64_t)R * SB * SB, nr, 0, nr, 0, nr);
-#pragma unroll
-    for (int j = 0; j < kStages; ++j) {
-      const int q = lo + j;
-      if (q < hi) cp_block(stage + j * SB * SB, F, m, r0, nr, SB * q, min(SB, k - SB * q));
-      cp_async_commit();
-    }
-    if (!started) {  // the unit's factor blocks are on their way; its vectors are the predecessor's
-      wait_previous();
-      started = true;
-    }
     T wrow[NR];
     if (fin && g == 0) {
 #pragma unroll
@@ -1820,36 +1873,43 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
             if (r < nr_rhs) tot[r] += __ldcg(my_part + (int64_t)c * SB * nr_rhs + i + SB * r);
       }
     };
-    // The flags of a front are set in chain order (the unit that sets flag q has
-    // waited for flag q - 1), so the newest flag of the range stands for all of
-    // them.  A unit other than a chain unit (final unit of a pivot row) waits for
-    // it on one thread and stages the y of all its blocks with one barrier; a
-    // chain unit checks it once and, unless it is set, takes its blocks as their
-    // flags appear.
+    // Every thread looks once for its share of the y of the unit's blocks.  If some are
+    // missing, a unit other than a chain unit (final unit of a pivot row) waits for all
+    // of them; a chain unit takes its blocks as they appear.
     const bool chain = fin && piv;
-    if (t == 0) {
-      int ready = 1;
-      if (lo < hi) {
-        if (!chain) wait_flag_backoff(flags + hi - 1, fa.err, 1024);
-        else ready = ld_acquire(flags + hi - 1) != 0;
+    auto y_of = [&](int e, bool wait) {  // entry e of [block][right-hand side][row]
+      const int c = e % SB, rr = (e / SB) % NR, q = lo + e / (SB * NR);
+      if (q >= hi || rr >= nr_rhs || c >= min(SB, k - SB * q)) return (T)0;
+      const T* p = mail + (int64_t)lo * SB * NR + e;
+      return wait ? wait_mail(p, fa.err) : read_mail(p);
+    };
+    bool have = true;
+    {
+      T v[kStageLoads<NR>];
+#pragma unroll
+      for (int j = 0; j < kStageLoads<NR>; ++j) v[j] = y_of(t + 256 * j, false);
+#pragma unroll
+      for (int j = 0; j < kStageLoads<NR>; ++j) {
+        const int e = t + 256 * j;
+        have = have && !empty_mail(v[j]);
+        if (e < (hi - lo) * SB * NR) ys[e / (SB * NR)][e % SB][(e / SB) % NR] = v[j];
       }
-      s_ready = ready;
     }
-    __syncthreads();
-    const bool staged = s_ready != 0;
-    if (staged && lo < hi) {
-      for (int e = t; e < (hi - lo) * SB * NR; e += 256) {
-        const int b = e / (SB * NR), c = (e / NR) % SB, r = e % NR;
-        const int q = lo + b;
-        ys[b][c][r] = (r < nr_rhs && c < min(SB, k - SB * q)) ? __ldcg(w + SB * q + c + (int64_t)r * m) : (T)0;
-      }
+    if (t == 0) s_tk[par ^ 1] = next;
+    const bool all = __syncthreads_and(have) != 0, staged = all || !chain;
+    ahead = s_tk[par ^ 1];
+    top_up();
+    if (!all && !chain) {
+      if (t == 0) wait_mail_backoff(mail + (int64_t)(hi - 1) * SB * NR, fa.err, 1024);
+      __syncthreads();
+      for (int e = t; e < (hi - lo) * SB * NR; e += 256)
+        ys[e / (SB * NR)][e % SB][(e / SB) % NR] = y_of(e, true);
       __syncthreads();
     }
     if (lo == hi) gather();
     for (int q = lo; q < hi; ++q) {
-      const int slot = (q - lo) % kStages;
       if (q == hi - 1) gather();
-      const T* blk = stage + slot * SB * SB + t;
+      const T* blk = stage + ring.take * SB * SB + t;
       if (!staged && t < SB) {
         // two warps wait for the block's values and bring them in for all
         const int wq = min(SB, k - SB * q);
@@ -1857,7 +1917,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
         for (int r = 0; r < NR; ++r)
           ys[q - lo][t][r] = (r < nr_rhs && t < wq) ? wait_mail(mail + (q * NR + r) * SB + t, fa.err) : (T)0;
       }
-      cp_async_wait<kStages - 1>();
+      ring.wait_oldest();
       if (!staged) __syncthreads();
       const T(*yb)[NR] = ys[q - lo];
 #pragma unroll
@@ -1866,10 +1926,10 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
 #pragma unroll
         for (int r = 0; r < NR; ++r) acc[r][e & 3] = fma(l, yb[g + 4 * e][r], acc[r][e & 3]);
       }
-      // the slot's values are in registers and used: refill it
-      const int qn = q + kStages;
-      if (qn < hi) cp_block(stage + slot * SB * SB, F, m, r0, nr, SB * qn, min(SB, k - SB * qn));
-      cp_async_commit();
+      // the slot's values are in registers and used: refill it (a link of the chain
+      // first finishes, its successor waits)
+      ring.pop();
+      if (q < hi - 1 || !chain) top_up();
     }
     // row totals: chunk partials (in order), then the four column groups
     T sum[NR];
@@ -1891,7 +1951,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
         if (i < nr) {
 #pragma unroll
           for (int r = 0; r < NR; ++r)
-            if (r < nr_rhs) w[r0 + i + (int64_t)r * m] -= tot[r] + sum[r];
+            if (r < nr_rhs) w[r0 + i + (int64_t)r * m] = wrow[r] - (tot[r] + sum[r]);
         }
       } else {
 #pragma unroll
@@ -1900,7 +1960,8 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
     }
     if (fin && piv) {
       // y_R = Dinv_R z: thread (i, g) sums its 16 columns, then the groups are added
-      cp_async_wait_all();
+      const T* dsm = stage + ring.take * SB * SB;
+      ring.wait_oldest();
       __syncthreads();
       T y4[NR][4];
 #pragma unroll
@@ -1930,13 +1991,10 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
           }
       }
     }
-    const bool publish = !fin || piv;
-    if (t == 0) s_tk[par ^ 1] = next;
     __syncthreads();
-    if (t == 0 && publish) {
-      if (fin) publish_flag(fa.flags + u.flag0 + R);
-      else publish_add(fa.counters + u.cnt);
-    }
+    if (t == 0 && !fin) publish_add(fa.counters + u.cnt);
+    if (chain) ring.pop();
+    top_up();
   }
   next_may_start();
   cp_async_wait_all();
@@ -1951,17 +2009,45 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
                                                     int64_t ldx, int nr_rhs, FusedArgs fa) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   T* stage = reinterpret_cast<T*>(sm_raw);
-  T* dsm = stage + kStages * SB * SB;
   __shared__ T red[2][SB][NR];  // per row half: column sums
   __shared__ T zs[SB][NR];      // y_p - sum, the input of the inverse
   __shared__ T xs[kUnitBlocks][SB][NR];  // x of the row blocks of the unit (when staged)
-  __shared__ int s_tk[2], s_ready;
+  __shared__ int s_tk[2];
   const int t = threadIdx.x, i = t & 63, g = t >> 6, lane = t & 31, half = (t >> 5) & 1;
   // column of the warp-reduced value this lane holds
   const int cl = g + 4 * ((lane >> 1) & 15);
   if (t == 0) s_tk[0] = atomicAdd(fa.ticket, 1);
   __syncthreads();
-  bool started = false;
+  // as in k_fwd_stream, with row blocks cR, cR - 1, ... clo of the column block at cc0
+  Ring ring;
+  int ahead = s_tk[0], cR = -1, clo = 0, cm = 0, ck = 0, cc0 = 0, cwc = 0;
+  const T *cF = L, *cD = nullptr;
+  auto top_up = [&]() {
+    while (ring.depth < kStages) {
+      if (cR < clo && cD == nullptr) {
+        if (ahead >= fa.count) break;
+        const Unit v = load_unit(fa.units, ahead);
+        ahead = INT_MAX;
+        cc0 = SB * v.R;
+        cwc = min(SB, v.k - cc0);
+        // rows farthest from the diagonal first (their x are known earliest)
+        cR = v.hi - 1, clo = v.lo, cm = v.m, ck = v.k;
+        cF = L + v.l_off;
+        if (v.fin != 0) cD = Dinv + v.dinv_off + (int64_t)v.R * SB * SB;
+      }
+      const bool blk = cR >= clo;
+      const int vpb = (ck + SB - 1) / SB;
+      const int r0 = cR < vpb ? SB * cR : ck + SB * (cR - vpb);
+      cp_block(stage + ring.free_slot() * SB * SB, blk ? cF : cD, blk ? cm : cwc, blk ? r0 : 0,
+               blk ? min(SB, (cR < vpb ? ck : cm) - r0) : cwc, blk ? cc0 : 0, cwc);
+      cp_async_commit();
+      ++ring.depth;
+      if (blk) --cR;
+      else cD = nullptr;
+    }
+  };
+  top_up();
+  wait_previous();  // the first blocks are on their way; the vectors are the predecessor's
   for (int par = 0;; par ^= 1) {
     const int tk = s_tk[par];
     if (tk >= fa.count) break;
@@ -1972,30 +2058,13 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
     const bool fin = u.fin != 0;
     const int pb = (k + SB - 1) / SB;
     const int c0 = SB * p, wc = min(SB, k - c0);
-    const T* F = L + u.l_off;
     T* w = W + u.w_off * nr_rhs;
-    const int* flags = fa.flags + u.flag0;
     T* mail = static_cast<T*>(fa.mail) + (int64_t)u.flag0 * SB * NR;
     auto rows_of = [&](int R, int& r0, int& nr) {
       r0 = (R < pb) ? SB * R : k + SB * (R - pb);
       nr = min(SB, (R < pb ? k : m) - r0);
     };
-    if (fin) cp_block(dsm, Dinv + u.dinv_off + (int64_t)p * SB * SB, wc, 0, wc, 0, wc);
-    // rows farthest from the diagonal first (their x are known earliest)
-#pragma unroll
-    for (int j = 0; j < kStages; ++j) {
-      const int R = hi - 1 - j;
-      if (R >= lo) {
-        int r0, nr;
-        rows_of(R, r0, nr);
-        cp_block(stage + j * SB * SB, F, m, r0, nr, c0, wc);
-      }
-      cp_async_commit();
-    }
-    if (!started) {  // the unit's factor blocks are on their way; its vectors are the predecessor's
-      wait_previous();
-      started = true;
-    }
+    const int pos = (fin && t < wc) ? rows[u.w_off + c0 + t] : 0;
     T wrow[NR];
     if (fin && t < SB) {
 #pragma unroll
@@ -2021,34 +2090,45 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
             if (r < nr_rhs) tot[r] += __ldcg(my_part + (int64_t)c * SB * nr_rhs + t + SB * r);
       }
     };
-    // Flags are set in chain order (last column first), so flag lo stands for
-    // every pivot row block of the range.  A chunk waits for it on one thread and
-    // stages x of all its row blocks with one barrier; the final unit (a link of
-    // the chain) checks it once and, unless it is set, stages only the update
-    // rows (no flag) and takes the pivot row blocks as their flags appear.
-    if (t == 0) {
-      int ready = 1;
-      if (lo < hi && lo < pb) {
-        if (!fin) wait_flag_backoff(flags + lo, fa.err, 1024);
-        else ready = ld_acquire(flags + lo) != 0;
+    // Every thread looks once for its share of the x of the unit's row blocks (those of
+    // update rows are there from the start).  If some are missing, a chunk waits for all
+    // of them; the final unit (a link of the chain) takes its pivot row blocks as they
+    // appear.
+    auto x_of = [&](int e, bool wait) {  // entry e of [block][right-hand side][row]
+      const int ii = e % SB, rr = (e / SB) % NR, R = lo + e / (SB * NR);
+      int r0, nr;
+      rows_of(R, r0, nr);
+      if (R >= hi || rr >= nr_rhs || ii >= nr) return (T)0;
+      if (R >= pb) return __ldcg(w + r0 + ii + (int64_t)rr * m);
+      const T* p = mail + (int64_t)lo * SB * NR + e;
+      return wait ? wait_mail(p, fa.err) : read_mail(p);
+    };
+    bool have = true;
+    {
+      T v[kStageLoads<NR>];
+#pragma unroll
+      for (int j = 0; j < kStageLoads<NR>; ++j) v[j] = x_of(t + 256 * j, false);
+#pragma unroll
+      for (int j = 0; j < kStageLoads<NR>; ++j) {
+        const int e = t + 256 * j;
+        have = have && (lo + e / (SB * NR) >= pb || !empty_mail(v[j]));
+        if (e < (hi - lo) * SB * NR) xs[e / (SB * NR)][e % SB][(e / SB) % NR] = v[j];
       }
-      s_ready = ready;
     }
-    __syncthreads();
-    const bool staged = s_ready != 0;
-    const int sfirst = staged ? lo : max(lo, pb);  // first staged row block
-    if (sfirst < hi) {
-      for (int e = t; e < (hi - sfirst) * SB * NR; e += 256) {
-        const int b = e / (SB * NR), ii = (e / NR) % SB, r = e % NR;
-        int r0, nr;
-        rows_of(sfirst + b, r0, nr);
-        xs[sfirst - lo + b][ii][r] = (r < nr_rhs && ii < nr) ? __ldcg(w + r0 + ii + (int64_t)r * m) : (T)0;
-      }
+    if (t == 0) s_tk[par ^ 1] = next;
+    const bool all = __syncthreads_and(have) != 0;
+    const int sfirst = all || !fin ? lo : max(lo, pb);  // first staged row block
+    ahead = s_tk[par ^ 1];
+    top_up();
+    if (!all && !fin) {
+      if (t == 0) wait_mail_backoff(mail + (int64_t)lo * SB * NR, fa.err, 1024);
+      __syncthreads();
+      for (int e = t; e < (hi - lo) * SB * NR; e += 256)
+        xs[e / (SB * NR)][e % SB][(e / SB) % NR] = x_of(e, true);
       __syncthreads();
     }
     if (lo == hi) gather();
     for (int R = hi - 1; R >= lo; --R) {
-      const int slot = (hi - 1 - R) % kStages;
       int r0, nr;
       rows_of(R, r0, nr);
       if (R == lo) gather();
@@ -2058,25 +2138,20 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
         for (int r = 0; r < NR; ++r)
           xs[R - lo][t][r] = (r < nr_rhs && t < nr) ? wait_mail(mail + (R * NR + r) * SB + t, fa.err) : (T)0;
       }
-      cp_async_wait<kStages - 1>();
+      ring.wait_oldest();
       if (R < sfirst) __syncthreads();
       T xv[NR];
 #pragma unroll
       for (int r = 0; r < NR; ++r) xv[r] = xs[R - lo][i][r];
-      const T* blk = stage + slot * SB * SB + t;
+      const T* blk = stage + ring.take * SB * SB + t;
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
         const T l = blk[e * 256];
 #pragma unroll
         for (int r = 0; r < NR; ++r) acc[r][e] = fma(l, xv[r], acc[r][e]);
       }
-      const int Rn = R - kStages;
-      if (Rn >= lo) {
-        int rn0, nrn;
-        rows_of(Rn, rn0, nrn);
-        cp_block(stage + slot * SB * SB, F, m, rn0, nrn, c0, wc);
-      }
-      cp_async_commit();
+      ring.pop();
+      if (R > lo || !fin) top_up();
     }
     // column totals: rows within the warp, then the two row halves
 #pragma unroll
@@ -2101,7 +2176,8 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
     if (fin) {
       // x_p = Dinv_p^T z: thread (i, g) forms D(i, c) z(i) for its 16 columns, then
       // the rows are added as above
-      cp_async_wait_all();
+      const T* dsm = stage + ring.take * SB * SB;
+      ring.wait_oldest();
       __syncthreads();
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
@@ -2116,7 +2192,6 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
       }
       __syncthreads();
       if (t < wc) {
-        const int pos = rows[u.w_off + c0 + t];
 #pragma unroll
         for (int r = 0; r < NR; ++r)
           if (r < nr_rhs) {
@@ -2127,12 +2202,10 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
           }
       }
     }
-    if (t == 0) s_tk[par ^ 1] = next;
     __syncthreads();
-    if (t == 0) {
-      if (fin) publish_flag(fa.flags + u.flag0 + p);
-      else publish_add(fa.counters + u.cnt);
-    }
+    if (t == 0 && !fin) publish_add(fa.counters + u.cnt);
+    if (fin) ring.pop();
+    top_up();
   }
   next_may_start();
   cp_async_wait_all();
