@@ -504,6 +504,11 @@ __device__ __forceinline__ void cp_async_elem(void* dst, const void* src, int sr
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(BYTES), "r"(src_bytes)
                : "memory");
 }
+template <int BYTES>
+__device__ __forceinline__ void cp_async_elem(void* dst, const void* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -1673,7 +1678,9 @@ __global__ void __launch_bounds__(256, 2) k_bwd_level(const T* __restrict__ L, c
 // one (two warps wait and bring the values into shared memory for the others) and any
 // other unit waits for all of them.  A link takes 1.45 us forward and 1.6 backward (6.3 and
 // 2.5 with a flag that every warp polls for itself).  Reading ahead and the single look in
-// place of a flag and a read took the 40^3-cell step's solve from 1.31 to 1.24 ms.  The four
+// place of a flag and a read took the 40^3-cell step's solve from 1.31 to 1.24 ms, and copies
+// of full blocks without a bounds check for each element (a warp spent 963 instructions on a
+// unit of the leaf level, most of them on addresses) to 1.19 ms.  The four
 // column groups (forward) or 64 rows (backward) of a block are combined once per unit, in a
 // fixed order, so results are deterministic.
 // ---------------------------------------------------------------------------
@@ -1685,12 +1692,21 @@ constexpr int kStages = 3;
 template <class T>
 __device__ __forceinline__ void cp_block(T* buf, const T* __restrict__ F, int64_t ld, int r0, int nr, int c0, int nc) {
   const int t = threadIdx.x, i = t & 63, g = t >> 6;
+  constexpr int E = (int)sizeof(T);
+  const T* src = F + (r0 + i) + (int64_t)(c0 + g) * ld;
+  const int64_t step = 4 * ld;
+  T* dst = buf + t;
+  if (nr == SB && nc == SB) {
 #pragma unroll
-  for (int e = 0; e < 16; ++e) {
-    const int c = g + 4 * e;
-    const bool ok = i < nr && c < nc;
-    const T* src = ok ? F + (r0 + i) + (int64_t)(c0 + c) * ld : F;
-    cp_async_elem<(int)sizeof(T)>(buf + e * 256 + t, src, ok ? (int)sizeof(T) : 0);
+    for (int e = 0; e < 16; ++e, src += step) cp_async_elem<E>(dst + e * 256, src);
+  } else {
+    const int last = i < nr ? nc - g : 0;  // 4 e < last: inside
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const bool ok = 4 * e < last;
+      cp_async_elem<E>(dst + e * 256, ok ? src : F, ok ? E : 0);
+      src += step;
+    }
   }
 }
 
@@ -1897,7 +1913,10 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
     }
     if (t == 0) s_tk[par ^ 1] = next;
     const bool all = __syncthreads_and(have) != 0, staged = all || !chain;
-    ahead = s_tk[par ^ 1];
+    // (a link that waits leaves the next unit's blocks until its own values are out: 499 in
+    // place of 581 us in the root front of an 80^3-cell model; backward, where a link's last
+    // blocks come late, the other way was the faster one, 505 in place of 542)
+    if (staged) ahead = s_tk[par ^ 1];
     top_up();
     if (!all && !chain) {
       if (t == 0) wait_mail_backoff(mail + (int64_t)(hi - 1) * SB * NR, fa.err, 1024);
@@ -1994,6 +2013,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_stream(const T* __restrict__ L, 
     __syncthreads();
     if (t == 0 && !fin) publish_add(fa.counters + u.cnt);
     if (chain) ring.pop();
+    if (!staged) ahead = s_tk[par ^ 1];
     top_up();
   }
   next_may_start();
