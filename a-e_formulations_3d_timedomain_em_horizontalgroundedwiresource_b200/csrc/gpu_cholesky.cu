@@ -3395,9 +3395,9 @@ void GpuCholesky::solve_with(const SolveSchedule& sc, const double* d_b, double*
 }
 
 // Times every candidate schedule for nrhs columns on the factor in `slot` (stream
-// s, CUDA events, the median of three solves after one warm-up each) with scratch
-// copies of zero right-hand sides, and keeps the fastest.  Run before the solve's
-// graph is captured, so the graph replays the chosen schedule.
+// s, CUDA events) with scratch copies of zero right-hand sides, and keeps the fastest:
+// the median of three solves after one warm-up, for those that are near the best.  Run
+// before the solve's graph is captured, so the graph replays the chosen schedule.
 std::string GpuCholesky::tune_solve(int nrhs, int64_t ld, cudaStream_t s, int slot) {
   std::vector<SolveSchedule> cand;
   for (int kind = 0; kind < 3; ++kind)
@@ -3422,22 +3422,39 @@ std::string GpuCholesky::tune_solve(int nrhs, int64_t ld, cudaStream_t s, int sl
   TDEM_CUDA_TRY(cudaEventCreate(&ev[0]));
   TDEM_CUDA_TRY(cudaEventCreate(&ev[1]));
   std::string err;
-  size_t best = 0;
-  for (size_t i = 0; i < cand.size() && err.empty(); ++i) {
-    solve_with(cand[i], tb, tb + (size_t)ld * nrhs, ld, nrhs, s, slot);  // warm-up
-    float t[3];
-    for (float& ti : t) {
-      cudaEventRecord(ev[0], s);
-      solve_with(cand[i], tb, tb + (size_t)ld * nrhs, ld, nrhs, s, slot);
-      cudaEventRecord(ev[1], s);
-      if (cudaEventSynchronize(ev[1]) != cudaSuccess || cudaEventElapsedTime(&ti, ev[0], ev[1]) != cudaSuccess) {
-        err = "CUDA: solve autotuner timing failed";
-        break;
+  auto time_one = [&](const SolveSchedule& c, float& ms) {
+    cudaEventRecord(ev[0], s);
+    solve_with(c, tb, tb + (size_t)ld * nrhs, ld, nrhs, s, slot);
+    cudaEventRecord(ev[1], s);
+    if (cudaEventSynchronize(ev[1]) != cudaSuccess || cudaEventElapsedTime(&ms, ev[0], ev[1]) != cudaSuccess)
+      err = "CUDA: solve autotuner timing failed";
+    return err.empty();
+  };
+  // Most likely the fastest first, so that the others are soon seen to be slower.
+  std::vector<size_t> order;
+  for (int kind : {2, 0, 1})
+    for (size_t i = 0; i < cand.size(); ++i)
+      if (cand[i].kind == kind) order.push_back(i);
+  bool any = false;
+  size_t best = order[0];
+  for (size_t i : order) {
+    // A candidate that is half as slow again as the best so far needs no second opinion.  Its
+    // first solve may include loading the kernels, some milliseconds at most.
+    constexpr float kClear = 1.5f, kLoad = 10.0f;
+    float first, t[3];
+    if (!time_one(cand[i], first)) break;
+    cand[i].ms = first;
+    if (!any || first < kClear * cand[best].ms + kLoad) {
+      if (!time_one(cand[i], t[0])) break;
+      cand[i].ms = t[0];
+      if (!any || t[0] < kClear * cand[best].ms) {
+        if (!time_one(cand[i], t[1]) || !time_one(cand[i], t[2])) break;
+        std::sort(t, t + 3);
+        cand[i].ms = t[1];
       }
     }
-    std::sort(t, t + 3);
-    cand[i].ms = t[1];
-    if (cand[i].ms < cand[best].ms) best = i;
+    if (!any || cand[i].ms < cand[best].ms) best = i;
+    any = true;
   }
   cudaEventDestroy(ev[0]);
   cudaEventDestroy(ev[1]);
