@@ -490,12 +490,12 @@ std::string TransientSolve::setup_device(cudaStream_t stream) {
   if (const char* oz = std::getenv("TDEM_OZAKI")) chol_->set_ozaki(oz[0] != '0');
   chol_->set_ozaki_timing(true);
   int slots = opt_.factor_slots;
-  // The integer-pipe trailing update holds 199 KB of shared memory and 168 x 320
-  // registers per CTA, so it cannot share an SM with a level-solve CTA; a
+  // The integer-pipe trailing update holds nearly all shared memory and most
+  // registers of an SM, so it cannot share an SM with a level-solve CTA; a
   // factorization ahead of use still fills the SMs its panel chain (one front's
   // 64-column steps at a time) leaves idle.  Measured at 80^3 (E-form, BDF2, 160
-  // steps): one slot 0.161 forward solves/s; two slots with the level solves kept
-  // to one CTA per SM 0.157, with their full two CTAs per SM 0.169.
+  // steps): one slot 0.221 forward solves/s, two 0.228 (with an earlier update kernel
+  // 0.161 and 0.169, and 0.157 with the level solves kept to one CTA per SM).
   const char* oz_env = std::getenv("TDEM_OZAKI");
   const bool oz_planned = sy_->oz_rows_max > 0 && factor_bytes() == 8 && !(oz_env && oz_env[0] == '0');
   if (slots == 0) {

@@ -2737,7 +2737,7 @@ std::string set_attributes() {
 // Where a level's first inner panel has kLeftTiles or more tiles to its right, the outer
 // panel goes left-looking instead: each inner panel takes all the finished ones of its outer
 // panel in one update just before it is factored, so its columns are read and written once
-// and not up to three times, and nothing is left to run beside the chain, which such a level
+// and not up to seven times, and nothing is left to run beside the chain, which such a level
 // hides anyway.  (80^3 cells, two factorizations and 20 steps: 853 ms without, 839 / 840.5 /
 // 843 / 850 ms from 148 / 296 / 592 / 1,184 tiles on; 40^3 200.1 / 199.9 / 200.2 / 200.3 / 200.4;
 // with every level left-looking 8^3 cells go from 1.78 to 1.93 ms.)

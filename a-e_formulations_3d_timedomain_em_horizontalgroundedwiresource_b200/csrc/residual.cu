@@ -10,7 +10,7 @@
 // Pass 2 (a warp per sum) adds the kResBlocks partials.  The row -> thread assignment and
 // every summation order are fixed, so repeated calls on the same data give bit-identical
 // norms.  (A warp per row, all lanes gathering and reducing one column after another,
-// was 4,205 us for 270,400 rows of 27 entries and 32 columns, 225 MB; this is 297 us, bound by
+// was 4,205 us for 270,400 rows of 27 entries and 32 columns, 225 MB; this is 253 us, bound by
 // the reads of x through L1 and L2.)
 #include <cuda.h>
 #include <cuda_runtime.h>

@@ -31,10 +31,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, HERE)
 PKG = "a-e_formulations_3d_timedomain_em_horizontalgroundedwiresource_b200"
 METRIC = "forward solves/s + p50/p99 latency, mixed vs FP64 GPU, ≤1e-5 rel. error"
-# k_oz_update, one launch of the 40^3 half-space (ncu --set full, profiles/k_oz_update_c1.md):
+# k_oz_update, one launch of the 40^3 half-space (ncu, profiles/k_oz_update_c1.md):
 # DRAM bytes read + written and 8-bit tensor ops of that launch
-OZ_CAPTURE_DRAM_BYTES = 342.647296e6 + 200.931328e6
-OZ_CAPTURE_OPS = 493753466880.0
+OZ_CAPTURE_DRAM_BYTES = 442.996992e6 + 175.569408e6
+OZ_CAPTURE_OPS = 351113576448.0
 
 
 # ---------------------------------------------------------------------------
@@ -451,7 +451,7 @@ def run_ours(args, world, rank, local):
                                           else "fallback 6650 GB/s (MEASURED_PEAKS.json absent)")}
             roof_oz = None
             if inf["ozaki_macs"] > 0 and oz_ms > 0:
-                # the integer tensor pipe: 8-bit multiply-adds of the digit products per launch
+                # the integer tensor pipe: 8-bit multiply-adds of the residue products per launch
                 # time; peak = twice the measured dense bf16 rate (B200's 8-bit dense rate is
                 # twice its bf16 rate)
                 bf16 = peaks.get("bf16_tflops")
@@ -464,7 +464,7 @@ def run_ours(args, world, rank, local):
                 # ops do
                 traffic = OZ_CAPTURE_DRAM_BYTES / OZ_CAPTURE_OPS * 2.0 * inf["ozaki_macs"]
                 roof_oz = {"bound": "tensor", "kernel": "k_oz_update (tcgen05 kind::i8, FP64 trailing updates by "
-                                                        "digit splitting; the dominant kernel)",
+                                                        "residues; the dominant kernel)",
                            "achieved": ach, "peak": pk, "unit": "TOP/s (int8)", "frac": ach / pk,
                            "ops_per_launch": 2.0 * inf["ozaki_macs"],
                            "launch": "all k_oz_update launches of one factorization",

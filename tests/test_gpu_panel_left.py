@@ -1,6 +1,6 @@
 """Factorization of levels with many tiles, whose inner panels take the outer panel's
 finished ones in one update just before they are factored: fronts without update rows
-(dense blocks of n pivots, one to three outer panels' remainders) and with them (a chain of
+(dense blocks of n pivots; the 600 end in a second outer panel with few tiles) and with them (a chain of
 coupled blocks), with more tiles than SMs on a level (and, with 100 blocks, fewer).  The
 blocks' own levels are followed by levels of fronts without rows, which launch nothing: what
 a launch of no blocks leaves behind would fail the next case's set-up."""
@@ -24,6 +24,7 @@ def _blocks(n, count, coupled, seed):
 
 
 @pytest.mark.parametrize("n,count,coupled", [(129, 150, False), (192, 100, False), (200, 80, False), (321, 60, False),
+                                             (600, 40, False),
                                              (66, 511, True), (100, 255, True)])
 def test_backward_error_of_many_fronts(pkg, n, count, coupled):
     D, E, d = _blocks(n, count, coupled, n)
