@@ -23,6 +23,7 @@
 #include <cstdio>
 #include <type_traits>
 
+#include "diag_tiles.h"
 #include "tc_update.h"
 
 namespace tdem {
@@ -215,12 +216,14 @@ __global__ void __launch_bounds__(256) k_potrf(T* __restrict__ L, Fronts f, cons
                                                int* __restrict__ err, const int* __restrict__ c0_of,
                                                T* __restrict__ dinv = nullptr,
                                                const int64_t* __restrict__ dinv_off = nullptr) {
-  constexpr int QB = 16, CB = 8, LD = P + 2;
+  constexpr int QB = kDiagQ, CB = kDiagCols, LD = kDiagLd;
+  static_assert(P == kDiagPanel && kDiagTilesMax <= 24, "eight warps, three tiles each");
   // A(r, c), r >= c: the block, then its factor L(r, c).  A(c, r), r > c: the inverse
   // X(r, c) from its block row on; its diagonal is xd (the reciprocals of the factor's).
   // Rows of 528 bytes: a thread's own row and the diagonal block go by 16-byte accesses.
-  // (CB rows more than the block: the last 16-row tile of an update may reach past it.)
-  __shared__ __align__(16) T A[P + CB][LD];
+  // (CB rows more than the block: the last 16-row tile of an update may reach past it,
+  // see diag_tiles.h.)
+  __shared__ __align__(16) T A[kDiagRows][LD];
   __shared__ T xd[P];
   __shared__ T tb[3][QB][QB + 1];  // sums of the inverse's block row
   const int s = fronts[blockIdx.x];
@@ -339,13 +342,13 @@ __global__ void __launch_bounds__(256) k_potrf(T* __restrict__ L, Fronts f, cons
     }
     __syncthreads();
     // rank-8 update of the lower triangle right of the columns, 16 x 8 tiles
-    const int n = (wp - o - CB + QB - 1) / QB, tiles = n * (n + 1);
+    const int tiles = diag_tiles(wp, o);
 #pragma unroll
     for (int it = 0; it < 3; ++it) {
       const int tile = warp + 8 * it;
       if (tile >= tiles) break;
-      const int bi = tile < 2 ? 0 : (tile < 6 ? 1 : (tile < 12 ? 2 : 3)), h = tile - bi * (bi + 1);
-      const int r0 = o + CB + QB * bi, c0 = o + CB + 8 * h;
+      const DiagTile dt = diag_tile(o, tile);
+      const int r0 = dt.r0, c0 = dt.c0;
       T u[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) u[i] = A[r0 + g + 8 * (i >> 1)][c0 + 2 * q4 + (i & 1)];
