@@ -52,7 +52,9 @@ struct Fronts {
 // predecessor in the stream still runs, and reads or writes nothing the predecessor (or
 // what came before it) touches until wait_previous returns, which is when the
 // predecessor's grid has ended and its writes are visible; next_may_start says when the
-// successor may be set up.  What is saved is the launch and the ramp between dependent
+// successor may be set up.  Vectors that the chain's kernels write (W, x, part) are no
+// const __restrict__ parameters of a dependent: that would let the compiler read them as
+// constant over its whole life, which includes the predecessor's.  What is saved is the launch and the ramp between dependent
 // kernels of a few microseconds, of which a time step of a small mesh has dozens.
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -983,8 +985,10 @@ __global__ void __launch_bounds__(kSolveRows) k_fwd_update(const T* __restrict__
   }
 }
 
+// (x is what the level above stored, maybe after this grid had started: neither const
+// __restrict__ nor read through a path that takes it for constant)
 template <class T>
-__global__ void k_bwd_init(T* __restrict__ W, const double* __restrict__ x, SolveArgs a,
+__global__ void k_bwd_init(T* __restrict__ W, const double* x, SolveArgs a,
                            const int* __restrict__ fronts, const int64_t* __restrict__ prefix, int count) {
   next_may_start();
   wait_previous();
@@ -997,7 +1001,7 @@ __global__ void k_bwd_init(T* __restrict__ W, const double* __restrict__ x, Solv
   const int pos = a.rows[a.rows_off[s] + i];
 #pragma unroll 4
   for (int r = kColChunk * blockIdx.y; r < min(a.nrhs, kColChunk * ((int)blockIdx.y + 1)); ++r)
-    w[i + (int64_t)r * m] = (T)x[pos + r * a.ld];
+    w[i + (int64_t)r * m] = (T)__ldcg(x + pos + r * a.ld);
 }
 
 // Partial sums of L[j1:m, panel]^T W[j1:m] over one row chunk.
