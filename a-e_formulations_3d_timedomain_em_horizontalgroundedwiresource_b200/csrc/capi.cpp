@@ -679,6 +679,20 @@ int pardiso_analyse(PardisoHandle* h, int64_t n, const long long* ia, const long
   h->hash = pattern_hash(n, ia, ja);
   return 0;
 }
+
+// Waits for the handle's stream and returns PARDISO's error for what the factorization or
+// the solve on it met.  Where a bounded wait of a kernel gave up (-5), factor and solution
+// are not valid and the flag stays with the factor: it is dropped, so that a phase 33 has
+// none to use and the next phase 12 starts with a new one.
+int pardiso_outcome(PardisoHandle* h) {
+  int pivot = 0, gave_up = 0;
+  if (!h->chol->read_status(h->stream, &pivot, &gave_up)) return -2;
+  if (gave_up) {
+    h->chol.reset();
+    return -5;
+  }
+  return pivot ? -4 : 0;
+}
 }  // namespace
 
 static void pardiso_impl(void* pt, const long long* mtype, const long long* phase, const long long* n,
@@ -739,11 +753,7 @@ static void pardiso_impl(void* pt, const long long* mtype, const long long* phas
     for (int64_t q = 0; q < h->nnz; ++q) lv[h->upper_to_lower[q]] = av[q];
     cudaMemcpyAsync(h->d_vals, lv.data(), sizeof(double) * h->nnz, cudaMemcpyHostToDevice, h->stream);
     h->chol->factor(h->d_vals, h->stream);
-    if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
-      *error = -2;
-      return;
-    }
-    if (h->chol->status(h->stream)) *error = -4;
+    *error = pardiso_outcome(h);
     return;
   }
   if (*phase == 33) {
@@ -777,14 +787,7 @@ static void pardiso_impl(void* pt, const long long* mtype, const long long* phas
         return;
       }
       h->chol->factor(h->d_vals, h->stream);
-      if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
-        *error = -2;
-        return;
-      }
-      if (h->chol->status(h->stream)) {
-        *error = -4;
-        return;
-      }
+      if ((*error = pardiso_outcome(h)) != 0) return;
     }
     // all columns in one copy, solved in blocks of the analysed right-hand-side count
     cudaMemcpyAsync(h->d_x, b, sizeof(double) * h->n * nr, cudaMemcpyHostToDevice, h->stream);
@@ -793,7 +796,9 @@ static void pardiso_impl(void* pt, const long long* mtype, const long long* phas
       h->chol->solve(h->d_x + h->n * r, h->d_x + h->n * r, h->n, cols, h->stream);
     }
     cudaMemcpyAsync(x, h->d_x, sizeof(double) * h->n * nr, cudaMemcpyDeviceToHost, h->stream);
-    if (cudaStreamSynchronize(h->stream) != cudaSuccess) *error = -2;
+    // (a pivot that phase 12 reported is no error of the solve)
+    const int r = pardiso_outcome(h);
+    if (r != -4) *error = r;
     return;
   }
   *error = -1;
@@ -822,6 +827,16 @@ void pardiso_64(void* pt, const long long* maxfct, const long long* mnum, const 
 }
 
 void mkl_set_num_threads(int) {}
+
+// For tests (not in tdem.h): marks the factor of the handle kept for pt as if a wait of the
+// level solves (1) or of the tensor-core update (2) had given up.
+int tdem_test_pardiso_gave_up(void* pt, int which) {
+  PardisoHandle* h = pardiso_lookup(pt);
+  if (!h || !h->chol) return -1;
+  cudaSetDevice(h->device);
+  h->chol->mark_gave_up(which, h->stream);
+  return 0;
+}
 
 int tdem_pardiso_handles(void) {
   std::lock_guard<std::mutex> lk(g_pardiso_mu);

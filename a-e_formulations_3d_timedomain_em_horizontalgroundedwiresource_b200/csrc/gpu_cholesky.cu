@@ -3551,4 +3551,18 @@ int GpuCholesky::solve_status(cudaStream_t s) {
   return h[0] ? 1 : (h[1] ? 2 : 0);
 }
 
+bool GpuCholesky::read_status(cudaStream_t s, int* pivot, int* gave_up) {
+  int h[3] = {0, 0, 0};
+  if (cudaMemcpyAsync(h, d_err_, sizeof h, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess)
+    return false;
+  *pivot = h[0];
+  *gave_up = h[1] ? 1 : (h[2] ? 2 : 0);
+  return true;
+}
+
+void GpuCholesky::mark_gave_up(int which, cudaStream_t s) {
+  if (which == 1 || which == 2) cudaMemsetAsync(d_err_ + which, 1, sizeof(int), s);
+}
+
 }  // namespace tdem

@@ -85,6 +85,10 @@ class GpuCholesky {
   // 0 = ok; 1 = a wait of the level solves gave up, 2 = a wait of the
   // tensor-core update gave up (results since setup are not valid).
   int solve_status(cudaStream_t stream);
+  // Both at once, behind everything on the stream: false when the stream failed.
+  bool read_status(cudaStream_t stream, int* pivot, int* gave_up);
+  // Records what a wait that gave up would (solve_status() values 1 and 2); for tests.
+  void mark_gave_up(int which, cudaStream_t stream);
   // FP32 factor: trailing updates on the tensor cores (3xTF32) or on the
   // CUDA cores (default).  Takes effect at setup().
   void set_tensor_core_update(bool on) { tc_update_ = on; }

@@ -348,7 +348,8 @@ void tdem_server_destroy(tdem_server* srv);
  * right-hand sides b -> x), phase -1 (release).  The handle lives in pt[0];
  * maxfct, mnum, perm, iparm and msglvl are accepted and ignored.  *error: 0 ok,
  * -1 bad input / unsupported phase or mtype, -2 out of memory or CUDA error,
- * -4 non-positive pivot.  Runs on CUDA device 0 unless TDEM_PARDISO_DEVICE is set.
+ * -4 non-positive pivot, -5 a wait between the device's kernels gave up (factor and
+ * solution are not valid; factorize again).  Runs on CUDA device 0 unless TDEM_PARDISO_DEVICE is set.
  * The reference zeroes pt before every phase 12 (pardiso_solver::init,
  * pardiso.cpp:43-58, 76): the handle is also kept by the address of pt, so a
  * phase 12 on a zeroed pt reuses the analysis, factor memory and stream made
