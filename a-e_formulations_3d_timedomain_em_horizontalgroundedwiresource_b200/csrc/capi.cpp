@@ -752,6 +752,7 @@ static void pardiso_impl(void* pt, const long long* mtype, const long long* phas
     const double* av = (const double*)a;
     for (int64_t q = 0; q < h->nnz; ++q) lv[h->upper_to_lower[q]] = av[q];
     cudaMemcpyAsync(h->d_vals, lv.data(), sizeof(double) * h->nnz, cudaMemcpyHostToDevice, h->stream);
+    h->chol->clear_pivot(h->stream);
     h->chol->factor(h->d_vals, h->stream);
     *error = pardiso_outcome(h);
     return;

@@ -3561,6 +3561,8 @@ bool GpuCholesky::read_status(cudaStream_t s, int* pivot, int* gave_up) {
   return true;
 }
 
+void GpuCholesky::clear_pivot(cudaStream_t s) { cudaMemsetAsync(d_err_, 0, sizeof(int), s); }
+
 void GpuCholesky::mark_gave_up(int which, cudaStream_t s) {
   if (which == 1 || which == 2) cudaMemsetAsync(d_err_ + which, 1, sizeof(int), s);
 }

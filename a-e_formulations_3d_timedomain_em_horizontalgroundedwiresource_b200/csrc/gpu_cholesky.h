@@ -87,6 +87,8 @@ class GpuCholesky {
   int solve_status(cudaStream_t stream);
   // Both at once, behind everything on the stream: false when the stream failed.
   bool read_status(cudaStream_t stream, int* pivot, int* gave_up);
+  // Forgets a reported pivot, for a factorization of other values.
+  void clear_pivot(cudaStream_t stream);
   // Records what a wait that gave up would (solve_status() values 1 and 2); for tests.
   void mark_gave_up(int which, cudaStream_t stream);
   // FP32 factor: trailing updates on the tensor cores (3xTF32) or on the
