@@ -84,6 +84,12 @@ __device__ __forceinline__ double tsqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float tsqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double trsqrt(double x) { return rsqrt(x); }
 __device__ __forceinline__ float trsqrt(float x) { return 1.0f / sqrtf(x); }
+// the upper word of a positive value, and of the least normal one: the reciprocal of a
+// smaller pivot may overflow (its square root's never does)
+__device__ __forceinline__ int upper_word(double x) { return __double2hiint(x); }
+__device__ __forceinline__ int upper_word(float x) { return __float_as_int(x); }
+template <class T>
+constexpr int kLeastNormal = std::is_same<T, double>::value ? 0x00100000 : 0x00800000;
 
 // ---------------------------------------------------------------------------
 // factorization kernels
@@ -293,10 +299,12 @@ __global__ void __launch_bounds__(256) k_potrf(T* __restrict__ L, Fronts f, cons
 #pragma unroll
       for (int c = 0; c < CB; ++c) x[c] = row[c];
       asm volatile("bar.sync 1, 64;" ::: "memory");  // both warps hold the block before its rows change
+      int least = INT_MAX;
 #pragma unroll
       for (int j = 0; j < CB; ++j) {
         const T d = M[j][j] > (T)0 ? M[j][j] : (T)1;
         dj[j] = d;
+        least = min(least, upper_word(d));
         const T rc = (T)1 / d;
         T u[CB];
 #pragma unroll
@@ -320,6 +328,33 @@ __global__ void __launch_bounds__(256) k_potrf(T* __restrict__ L, Fronts f, cons
         const T inv = trsqrt(dj[c]);
         x[c] *= inv;
         if (t == o) xd[o + c] = inv;
+      }
+      if (least < kLeastNormal<T>) {
+        // A subnormal pivot (the same finding in all 64 threads, which hold the same block):
+        // all of it again, every column scaled by its pivot's root before it is used.
+#pragma unroll
+        for (int i = 0; i < CB; ++i)
+#pragma unroll
+          for (int c = 0; c <= i; ++c) M[i][c] = A[o + i][o + c];
+#pragma unroll
+        for (int c = 0; c < CB; ++c) x[c] = row[c];
+        asm volatile("bar.sync 1, 64;" ::: "memory");  // as above
+#pragma unroll
+        for (int j = 0; j < CB; ++j) {
+          const T d = M[j][j] > (T)0 ? M[j][j] : (T)1, inv = trsqrt(d);
+          mine = t == o + j ? d : mine;
+          if (t == o) xd[o + j] = inv;
+          x[j] *= inv;
+#pragma unroll
+          for (int i = j + 1; i < CB; ++i) {
+            M[i][j] *= inv;
+            x[i] = fma(-x[j], M[i][j], x[i]);
+          }
+#pragma unroll
+          for (int i = j + 1; i < CB; ++i)
+#pragma unroll
+            for (int c = j + 1; c <= i; ++c) M[i][c] = fma(-M[i][j], M[c][j], M[i][c]);
+        }
       }
       const T root = tsqrt(mine);
       if (t >= o && t < wp) {
