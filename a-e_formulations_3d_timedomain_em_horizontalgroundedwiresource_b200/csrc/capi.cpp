@@ -794,7 +794,11 @@ static void pardiso_impl(void* pt, const long long* mtype, const long long* phas
     cudaMemcpyAsync(h->d_x, b, sizeof(double) * h->n * nr, cudaMemcpyHostToDevice, h->stream);
     for (int r = 0; r < nr; r += h->solve_cols) {
       const int cols = std::min(h->solve_cols, nr - r);
-      h->chol->solve(h->d_x + h->n * r, h->d_x + h->n * r, h->n, cols, h->stream);
+      if (!h->chol->solve(h->d_x + h->n * r, h->d_x + h->n * r, h->n, cols, h->stream).empty()) {
+        cudaStreamSynchronize(h->stream);  // b may be on its way still
+        *error = -2;
+        return;
+      }
     }
     cudaMemcpyAsync(x, h->d_x, sizeof(double) * h->n * nr, cudaMemcpyDeviceToHost, h->stream);
     // (a pivot that phase 12 reported is no error of the solve)

@@ -1079,7 +1079,8 @@ std::string TransientSolve::time_step(bool block, int reps, double* ms) {
     for (int j = 0; j < npls_; ++j) {
       launch_history_rhs(d_rowptr_, d_col_, d_C_, u + j * n, u + j * n, 1.0, 0.0, d_S_ + j * n, 0.0, d_bound_, n_,
                          1, d_rhs_ + j * n, nullptr, s_);
-      chol_->solve(d_rhs_ + j * n, d_x_ + j * n, n_, 1, s_, slot_);
+      const std::string se = chol_->solve(d_rhs_ + j * n, d_x_ + j * n, n_, 1, s_, slot_);
+      if (!se.empty()) return se;
     }
     return "";
   };

@@ -60,7 +60,7 @@ __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.w
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... P, class... A>
-void launch_next(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
+cudaError_t launch_next(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
@@ -71,7 +71,17 @@ void launch_next(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, c
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+// The same without the attribute: it starts when the stream has ended what came before.
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 // Element (i, c), i >= c, of a split front.
@@ -2913,49 +2923,55 @@ int launch_factor(const Symbolic& sy, T* L, T* U, const double* vals, const int6
   return launches;
 }
 
+// What a solve put on its stream: the kernels, and the first error of a launch or a memset
+// (in a captured solve a failed one would be a missing node).
+struct Launched {
+  int kernels = 0;
+  cudaError_t err = cudaSuccess;
+  void check(cudaError_t e) {
+    if (err == cudaSuccess) err = e;
+  }
+  void add(cudaError_t e) {
+    check(e);
+    ++kernels;
+  }
+};
+
 template <class T>
-int launch_solve(const Symbolic& sy, const T* L, T* W, T* part, const double* b, double* x, SolveArgs a,
-                 const Kids& kids, const int* tasks, const int64_t* prefix,
-                 cudaStream_t s) {
-  int launches = 0;
+Launched launch_solve(const Symbolic& sy, const T* L, T* W, T* part, const double* b, double* x, SolveArgs a,
+                      const Kids& kids, const int* tasks, const int64_t* prefix, cudaStream_t s) {
+  Launched done;
   const size_t ysm = sizeof(T) * P * a.nrhs;
   for (const LevelPlan& lp : sy.levels) {
     if (lp.assemble.ctas == 0) continue;  // only fronts without rows
-    k_fwd_gather<T><<<front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s>>>(W, b, a, kids, tasks + lp.assemble.off,
-                                                                     prefix + lp.assemble.pre, lp.assemble.count);
-    ++launches;
+    done.add(launch_after(k_fwd_gather<T>, front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s, W, b, a, kids,
+             tasks + lp.assemble.off, prefix + lp.assemble.pre, lp.assemble.count));
     for (const PanelStep& ps : lp.panels) {
-      k_fwd_diag<T><<<ps.potrf.count, 256, ysm, s>>>(L, W, a, tasks + ps.potrf.off, ps.j0);
-      ++launches;
+      done.add(launch_after(k_fwd_diag<T>, ps.potrf.count, 256, ysm, s, L, W, a, tasks + ps.potrf.off, ps.j0));
       if (ps.solve_upd.ctas > 0) {
-        k_fwd_update<T><<<grid_of(ps.solve_upd.ctas), kSolveRows, ysm, s>>>(
-            L, W, a, tasks + ps.solve_upd.off, prefix + ps.solve_upd.pre, ps.solve_upd.count, ps.j0);
-        ++launches;
+        done.add(launch_after(k_fwd_update<T>, grid_of(ps.solve_upd.ctas), kSolveRows, ysm, s, L, W, a,
+                 tasks + ps.solve_upd.off, prefix + ps.solve_upd.pre, ps.solve_upd.count, ps.j0));
       }
     }
   }
   for (int l = (int)sy.levels.size() - 1; l >= 0; --l) {
     const LevelPlan& lp = sy.levels[l];
     if (lp.assemble.ctas == 0) continue;  // only fronts without rows
-    k_bwd_init<T><<<front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s>>>(W, x, a, tasks + lp.assemble.off,
-                                                                   prefix + lp.assemble.pre, lp.assemble.count);
-    ++launches;
+    done.add(launch_after(k_bwd_init<T>, front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s, W, x, a,
+             tasks + lp.assemble.off, prefix + lp.assemble.pre, lp.assemble.count));
     for (int p = (int)lp.panels.size() - 1; p >= 0; --p) {
       const PanelStep& ps = lp.panels[p];
       if (ps.solve_upd.ctas > 0) {
-        k_bwd_partial<T><<<grid_of(ps.solve_upd.ctas), kSolveRows, 0, s>>>(
-            L, W, a, part, tasks + ps.solve_upd.off, prefix + ps.solve_upd.pre, ps.solve_upd.count, ps.j0);
-        ++launches;
+        done.add(launch_after(k_bwd_partial<T>, grid_of(ps.solve_upd.ctas), kSolveRows, 0, s, L, W, a, part,
+                 tasks + ps.solve_upd.off, prefix + ps.solve_upd.pre, ps.solve_upd.count, ps.j0));
       }
-      k_bwd_diag<T><<<ps.potrf.count, 256, ysm, s>>>(L, W, a, part, tasks + ps.solve_upd.off,
-                                                      prefix + ps.solve_upd.pre, ps.j0);
-      ++launches;
+      done.add(launch_after(k_bwd_diag<T>, ps.potrf.count, 256, ysm, s, L, W, a, part, tasks + ps.solve_upd.off,
+               prefix + ps.solve_upd.pre, ps.j0));
     }
-    k_bwd_store<T><<<grid_of(lp.assemble.ctas), kSolveRows, 0, s>>>(W, x, a, tasks + lp.assemble.off,
-                                                                    prefix + lp.assemble.pre, lp.assemble.count);
-    ++launches;
+    done.add(launch_after(k_bwd_store<T>, grid_of(lp.assemble.ctas), kSolveRows, 0, s, W, x, a,
+             tasks + lp.assemble.off, prefix + lp.assemble.pre, lp.assemble.count));
   }
-  return launches;
+  return done;
 }
 
 // ints of one group's tickets, flags and counters
@@ -2989,7 +3005,7 @@ inline int col_groups(const LevelPlan& lp, int nrhs) {
 template <class T, int RPT, bool STREAM, bool MR = false>
 void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T* part, const double* b, double* x,
                          SolveArgs a, const Kids& kids, const int* tasks,
-                         const int64_t* prefix, FusedArgs fa, int* sync, const int (&resident)[2], int& launches,
+                         const int64_t* prefix, FusedArgs fa, int* sync, const int (&resident)[2], Launched& done,
                          cudaStream_t s) {
   static_assert(!MR || std::is_same<T, double>::value, "the many-column persistent kernels are FP64");
   const int nlev = (int)sy.levels.size();
@@ -2998,9 +3014,9 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
   int* bflags = fflags + sy.n_flags;
   fa.counters = bflags + sy.n_flags;
   fa.stride = sync_ints(sy);
-  cudaMemsetAsync(sync, 0, sizeof(int) * (size_t)(fa.stride * (MR ? max_col_groups(a.nrhs) : 1)), s);
+  done.check(cudaMemsetAsync(sync, 0, sizeof(int) * (size_t)(fa.stride * (MR ? max_col_groups(a.nrhs) : 1)), s));
   const size_t mail = STREAM ? sizeof(T) * (size_t)sy.n_flags * SB * RPT : 0;  // one direction's
-  if constexpr (STREAM) cudaMemsetAsync(fa.mail, 0xFF, 2 * mail, s);
+  if constexpr (STREAM) done.check(cudaMemsetAsync(fa.mail, 0xFF, 2 * mail, s));
   const size_t ysm = STREAM ? stream_smem<T>() : (MR ? mr_smem() : sizeof(T) * SB * ys_ld(a.nrhs));
   auto grid = [&](int64_t count, int dir) {
     return (STREAM || MR) ? (unsigned)std::min<int64_t>(count, resident[dir]) : grid_of(count);
@@ -3008,9 +3024,8 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
   for (int l = 0; l < nlev; ++l) {
     const LevelPlan& lp = sy.levels[l];
     if (lp.assemble.ctas == 0) continue;  // only fronts without rows
-    launch_next(k_fwd_gather<T>, front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s, W, b, a, kids, tasks + lp.assemble.off,
-                                                                     prefix + lp.assemble.pre, lp.assemble.count);
-    ++launches;
+    done.add(launch_next(k_fwd_gather<T>, front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s, W, b, a, kids,
+             tasks + lp.assemble.off, prefix + lp.assemble.pre, lp.assemble.count));
     if (lp.fwd_count == 0) continue;
     FusedArgs f = fa;
     f.units = fa.units + (int64_t)kUnitInts * lp.fwd_off;
@@ -3021,24 +3036,22 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
       const int groups = col_groups(lp, a.nrhs);
       f.cols = (a.nrhs + groups - 1) / groups;
       auto go = [&](auto kernel) {
-        launch_next(kernel, dim3((unsigned)std::min<int64_t>(lp.fwd_count, std::max(1, resident[0] / groups)),
-                                 (unsigned)groups), 256, ysm, s, L, Dinv, W, part, a.nrhs, f);
+        done.add(launch_next(kernel, dim3((unsigned)std::min<int64_t>(lp.fwd_count, std::max(1,
+                 resident[0] / groups)), (unsigned)groups), 256, ysm, s, L, Dinv, W, part, a.nrhs, f));
       };
       f.cols <= 4 ? go(k_fwd_mrhs<1>) : f.cols <= 8 ? go(k_fwd_mrhs<2>) : f.cols <= 16 ? go(k_fwd_mrhs<4>)
                                                                                      : go(k_fwd_mrhs<8>);
     }
     else if constexpr (STREAM)
-      launch_next(k_fwd_stream<T, RPT>, grid(lp.fwd_count, 0), 256, ysm, s, L, Dinv, W, part, a.nrhs, f);
+      done.add(launch_next(k_fwd_stream<T, RPT>, grid(lp.fwd_count, 0), 256, ysm, s, L, Dinv, W, part, a.nrhs, f));
     else
-      launch_next(k_fwd_level<T, RPT>, grid(lp.fwd_count, 0), 256, ysm, s, L, Dinv, W, part, a.nrhs, f);
-    ++launches;
+      done.add(launch_next(k_fwd_level<T, RPT>, grid(lp.fwd_count, 0), 256, ysm, s, L, Dinv, W, part, a.nrhs, f));
   }
   for (int l = nlev - 1; l >= 0; --l) {
     const LevelPlan& lp = sy.levels[l];
     if (lp.assemble.ctas == 0) continue;  // only fronts without rows
-    launch_next(k_bwd_init<T>, front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s, W, x, a, tasks + lp.assemble.off,
-                                                                   prefix + lp.assemble.pre, lp.assemble.count);
-    ++launches;
+    done.add(launch_next(k_bwd_init<T>, front_grid(lp.assemble.ctas, a.nrhs), kSolveRows, 0, s, W, x, a,
+             tasks + lp.assemble.off, prefix + lp.assemble.pre, lp.assemble.count));
     if (lp.bwd_count == 0) continue;
     FusedArgs f = fa;
     f.units = fa.units + (int64_t)kUnitInts * lp.bwd_off;
@@ -3050,28 +3063,30 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
       const int groups = col_groups(lp, a.nrhs);
       f.cols = (a.nrhs + groups - 1) / groups;
       auto go = [&](auto kernel) {
-        launch_next(kernel, dim3((unsigned)std::min<int64_t>(lp.bwd_count, std::max(1, resident[1] / groups)),
-                                 (unsigned)groups), 256, ysm, s, L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
+        done.add(launch_next(kernel, dim3((unsigned)std::min<int64_t>(lp.bwd_count, std::max(1,
+                 resident[1] / groups)), (unsigned)groups), 256, ysm, s, L, Dinv, W, part, x, a.rows, a.ld, a.nrhs,
+                 f));
       };
       f.cols <= 4 ? go(k_bwd_mrhs<1>) : f.cols <= 8 ? go(k_bwd_mrhs<2>) : f.cols <= 16 ? go(k_bwd_mrhs<4>)
                                                                                      : go(k_bwd_mrhs<8>);
     }
     else if constexpr (STREAM)
-      launch_next(k_bwd_stream<T, RPT>, grid(lp.bwd_count, 1), 256, ysm, s, L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
+      done.add(launch_next(k_bwd_stream<T, RPT>, grid(lp.bwd_count, 1), 256, ysm, s, L, Dinv, W, part, x, a.rows,
+               a.ld, a.nrhs, f));
     else
-      launch_next(k_bwd_level<T, RPT>, grid(lp.bwd_count, 1), 256, ysm, s, L, Dinv, W, part, x, a.rows, a.ld, a.nrhs, f);
-    ++launches;
+      done.add(launch_next(k_bwd_level<T, RPT>, grid(lp.bwd_count, 1), 256, ysm, s, L, Dinv, W, part, x, a.rows,
+               a.ld, a.nrhs, f));
   }
 }
 
 template <class T>
-int launch_solve_fused(const Symbolic& sy, const T* L, const T* Dinv, T* W, T* part, const double* b, double* x,
+Launched launch_solve_fused(const Symbolic& sy, const T* L, const T* Dinv, T* W, T* part, const double* b, double* x,
                        SolveArgs a, const Kids& kids, const int* tasks,
                        const int64_t* prefix, FusedArgs fa, int* sync, const int (&resident)[2][2], cudaStream_t s) {
-  int launches = 0;
+  Launched done;
 #define TDEM_LEVELS(R, ST, RES) \
   launch_level_solves<T, R, ST>(sy, L, Dinv, W, part, b, x, a, kids, tasks, prefix, fa, sync, RES, \
-                                launches, s)
+                                done, s)
   if (a.nrhs == 1)
     TDEM_LEVELS(1, true, resident[0]);
   else if (a.nrhs == 2)
@@ -3087,17 +3102,17 @@ int launch_solve_fused(const Symbolic& sy, const T* L, const T* Dinv, T* W, T* p
   else
     TDEM_LEVELS(16, false, resident[0]);
 #undef TDEM_LEVELS
-  return launches;
+  return done;
 }
 
 // The persistent many-column level solves (FP64, 3 <= nrhs <= 32).
-int launch_solve_mr(const Symbolic& sy, const double* L, const double* Dinv, double* W, double* part, const double* b,
+Launched launch_solve_mr(const Symbolic& sy, const double* L, const double* Dinv, double* W, double* part, const double* b,
                     double* x, SolveArgs a, const Kids& kids, const int* tasks, const int64_t* prefix, FusedArgs fa, int* sync, const int (&resident)[2],
                     cudaStream_t s) {
-  int launches = 0;
+  Launched done;
   launch_level_solves<double, 8, false, true>(sy, L, Dinv, W, part, b, x, a, kids, tasks, prefix, fa, sync, resident,
-                                              launches, s);
-  return launches;
+                                              done, s);
+  return done;
 }
 
 // Resident CTAs of the persistent many-column kernels ([forward, backward]).
@@ -3400,26 +3415,30 @@ SolveSchedule GpuCholesky::schedule_for(int nrhs) const {
   return d;
 }
 
-void GpuCholesky::solve(const double* d_b, double* d_x, int64_t ld, int nrhs, cudaStream_t s, int slot) {
-  solve_with(schedule_for(nrhs), d_b, d_x, ld, nrhs, s, slot);
+std::string GpuCholesky::solve(const double* d_b, double* d_x, int64_t ld, int nrhs, cudaStream_t s, int slot) {
+  const cudaError_t e = solve_with(schedule_for(nrhs), d_b, d_x, ld, nrhs, s, slot);
+  if (e == cudaSuccess) return "";
+  cudaGetLastError();  // told here
+  return std::string("CUDA: launches of a solve: ") + cudaGetErrorString(e);
 }
 
-void GpuCholesky::solve_with(const SolveSchedule& sc, const double* d_b, double* d_x, int64_t ld, int nrhs,
-                             cudaStream_t s, int slot) {
+cudaError_t GpuCholesky::solve_with(const SolveSchedule& sc, const double* d_b, double* d_x, int64_t ld, int nrhs,
+                                    cudaStream_t s, int slot) {
   const Kids kids{d_kid_ptr_, d_kid_list_, d_inv_off_, d_inv_};
   if (sc.split > 1 && nrhs > 1) {
     // column groups one after another (each its own complete solve)
     const int per = (nrhs + sc.split - 1) / sc.split;
     SolveSchedule one = sc;
     one.split = 1;
-    int total = 0;
+    Launched all;
     for (int c = 0; c < nrhs; c += per) {
-      solve_with(one, d_b + (int64_t)c * ld, d_x + (int64_t)c * ld, ld, std::min(per, nrhs - c), s, slot);
-      total += launches_solve_;
+      all.check(solve_with(one, d_b + (int64_t)c * ld, d_x + (int64_t)c * ld, ld, std::min(per, nrhs - c), s, slot));
+      all.kernels += launches_solve_;
     }
-    launches_solve_ = total;
-    return;
+    launches_solve_ = all.kernels;
+    return all.err;
   }
+  Launched done;
   SolveArgs a{d_l_off_, d_w_off_, d_m_, d_k_, d_rows_off_, d_rows_, nrhs, ld};
   const void* Lp = d_L_[slot];
   const void* Dp = d_dinv_[slot];
@@ -3428,12 +3447,9 @@ void GpuCholesky::solve_with(const SolveSchedule& sc, const double* d_b, double*
     int res[2];
     for (int d = 0; d < 2; ++d)
       res[d] = solve_ctas_cap_ > 0 ? std::min(resident_mr_[d], solve_ctas_cap_ * sms_) : resident_mr_[d];
-    launches_solve_ = launch_solve_mr(sy_, (const double*)Lp, (const double*)Dp, (double*)d_W_, (double*)d_spart_,
-                                      d_b, d_x, a, kids, d_tasks_, d_prefix_, fa, d_sync_,
-                                      res, s);
-    return;
-  }
-  if (sc.kind != 1) {
+    done = launch_solve_mr(sy_, (const double*)Lp, (const double*)Dp, (double*)d_W_, (double*)d_spart_,
+                           d_b, d_x, a, kids, d_tasks_, d_prefix_, fa, d_sync_, res, s);
+  } else if (sc.kind != 1) {
     FusedArgs fa{d_units_, 0, nullptr, nullptr, nullptr, d_err_ + 1};
     fa.mail = d_mail_;
     int res[2][2];
@@ -3441,19 +3457,20 @@ void GpuCholesky::solve_with(const SolveSchedule& sc, const double* d_b, double*
       for (int d = 0; d < 2; ++d)
         res[j][d] = solve_ctas_cap_ > 0 ? std::min(resident_[j][d], solve_ctas_cap_ * sms_) : resident_[j][d];
     if (elem_ == 4)
-      launches_solve_ = launch_solve_fused<float>(sy_, (const float*)Lp, (const float*)Dp, (float*)d_W_,
-                                                  (float*)d_spart_, d_b, d_x, a, kids, d_tasks_, d_prefix_, fa, d_sync_, res, s);
+      done = launch_solve_fused<float>(sy_, (const float*)Lp, (const float*)Dp, (float*)d_W_, (float*)d_spart_, d_b,
+                                       d_x, a, kids, d_tasks_, d_prefix_, fa, d_sync_, res, s);
     else
-      launches_solve_ = launch_solve_fused<double>(sy_, (const double*)Lp, (const double*)Dp, (double*)d_W_,
-                                                   (double*)d_spart_, d_b, d_x, a, kids, d_tasks_, d_prefix_, fa, d_sync_, res, s);
-    return;
+      done = launch_solve_fused<double>(sy_, (const double*)Lp, (const double*)Dp, (double*)d_W_, (double*)d_spart_,
+                                        d_b, d_x, a, kids, d_tasks_, d_prefix_, fa, d_sync_, res, s);
+  } else if (elem_ == 4) {
+    done = launch_solve<float>(sy_, (const float*)Lp, (float*)d_W_, (float*)d_part_, d_b, d_x, a, kids, d_tasks_,
+                               d_prefix_, s);
+  } else {
+    done = launch_solve<double>(sy_, (const double*)Lp, (double*)d_W_, (double*)d_part_, d_b, d_x, a, kids, d_tasks_,
+                                d_prefix_, s);
   }
-  if (elem_ == 4)
-    launches_solve_ = launch_solve<float>(sy_, (const float*)Lp, (float*)d_W_, (float*)d_part_, d_b, d_x, a,
-                                          kids, d_tasks_, d_prefix_, s);
-  else
-    launches_solve_ = launch_solve<double>(sy_, (const double*)Lp, (double*)d_W_, (double*)d_part_, d_b, d_x, a,
-                                           kids, d_tasks_, d_prefix_, s);
+  launches_solve_ = done.kernels;
+  return done.err;
 }
 
 // Times every candidate schedule for nrhs columns on the factor in `slot` (stream
@@ -3486,9 +3503,9 @@ std::string GpuCholesky::tune_solve(int nrhs, int64_t ld, cudaStream_t s, int sl
   std::string err;
   auto time_one = [&](const SolveSchedule& c, float& ms) {
     cudaEventRecord(ev[0], s);
-    solve_with(c, tb, tb + (size_t)ld * nrhs, ld, nrhs, s, slot);
+    const cudaError_t le = solve_with(c, tb, tb + (size_t)ld * nrhs, ld, nrhs, s, slot);
     cudaEventRecord(ev[1], s);
-    if (cudaEventSynchronize(ev[1]) != cudaSuccess || cudaEventElapsedTime(&ms, ev[0], ev[1]) != cudaSuccess)
+    if (le != cudaSuccess || cudaEventSynchronize(ev[1]) != cudaSuccess || cudaEventElapsedTime(&ms, ev[0], ev[1]) != cudaSuccess)
       err = "CUDA: solve autotuner timing failed";
     return err.empty();
   };
@@ -3545,8 +3562,13 @@ std::string GpuCholesky::solve_graph(const double* d_b, double* d_x, int64_t ld,
     }
     cudaGraph_t g = nullptr;
     TDEM_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    solve(d_b, d_x, ld, nrhs, s, slot);
-    TDEM_CUDA_TRY(cudaStreamEndCapture(s, &g));
+    const std::string le = solve(d_b, d_x, ld, nrhs, s, slot);
+    const cudaError_t ce = cudaStreamEndCapture(s, &g);
+    if (!le.empty()) {  // the graph lacks a node
+      if (g) cudaGraphDestroy(g);
+      return le;
+    }
+    TDEM_CUDA_TRY(ce);
     const cudaError_t ie = cudaGraphInstantiate(&sg.exec, g, 0);
     cudaGraphDestroy(g);
     if (ie != cudaSuccess) {

@@ -72,7 +72,8 @@ class GpuCholesky {
   // arrays with leading dimension ld (positions given by perm_to_vec); x rows
   // not covered by the system are left untouched.  b and x may alias.  Solves
   // share their work vectors: they must not run concurrently with each other.
-  void solve(const double* d_b, double* d_x, int64_t ld, int nrhs, cudaStream_t stream, int slot = 0);
+  // Returns what a launch met ("" where all were made).
+  std::string solve(const double* d_b, double* d_x, int64_t ld, int nrhs, cudaStream_t stream, int slot = 0);
   // Same as solve(), replayed from a CUDA graph captured on first use for these
   // buffers and slot (the factor values may change between calls; the pointers
   // may not).
@@ -155,8 +156,8 @@ class GpuCholesky {
   SolveSchedule forced_;
   std::vector<std::pair<int, SolveSchedule>> tuned_;  // (column count, chosen schedule)
   std::vector<std::pair<int, std::vector<SolveSchedule>>> tune_log_;  // every candidate measured
-  void solve_with(const SolveSchedule& sc, const double* d_b, double* d_x, int64_t ld, int nrhs, cudaStream_t s,
-                  int slot);
+  cudaError_t solve_with(const SolveSchedule& sc, const double* d_b, double* d_x, int64_t ld, int nrhs,
+                         cudaStream_t s, int slot);
   std::string tune_solve(int nrhs, int64_t ld, cudaStream_t s, int slot);
   int elem_ = 8;                 // bytes per held factor entry and solve value (8 = FP64, 4 = FP32)
   int fac_elem_ = 8;             // bytes per entry of the factorization's arithmetic

@@ -484,7 +484,9 @@ std::string solve_stationary(const std::string& dir, int device, StationaryTimes
     STAT_CUDA(cudaMemcpyAsync(db.p, rhs.data(), sizeof(double) * (size_t)n * ncol, cudaMemcpyHostToDevice, st));
     for (int c0 = 0; c0 < ncol; c0 += nrhs_max) {
       const int nc = std::min(nrhs_max, ncol - c0);
-      chol.solve((const double*)db.p + (size_t)c0 * n, (double*)dx.p + (size_t)c0 * n, n, nc, st);
+      const std::string se =
+          chol.solve((const double*)db.p + (size_t)c0 * n, (double*)dx.p + (size_t)c0 * n, n, nc, st);
+      if (!se.empty()) return se;
     }
     STAT_CUDA(cudaGetLastError());
     out.resize((size_t)n * ncol);
