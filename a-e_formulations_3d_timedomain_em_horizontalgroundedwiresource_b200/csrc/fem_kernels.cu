@@ -12,6 +12,7 @@
 #include "fem_kernels.h"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace tdem {
 namespace {
@@ -160,6 +161,14 @@ __global__ void k_history_rhs(const int64_t* __restrict__ rowptr, const int* __r
   }
 }
 
+// Several sources, few values (rows x sources up to this): one launch that forms the
+// combination of the layers on the way, where a launch of its own costs more.  (us, warm L2,
+// one launch / two; 33 entries a row: 1,536 rows and 2 sources 7.5 / 11.6, 8 10.5 / 15.6, 32
+// 21 / 27; 6,591 rows and 2 7.6 / 12.1, 8 12.7 / 16.5, 16 18.7 / 21.6, 32 33 / 30; 12,288 rows
+// and 4 13.3 / 13.9, 5 18.9 / 16.6; 24,000 rows and 2 12.9 / 13.4, 3 18.9 / 14.5.  A warp a row
+// with column-major gathers took 7.3, 9.0, 17; 10.5, 13, 19, 31; 16.8, 16.9; 23, 25.)
+constexpr int64_t kDirectValues = 56 * 1024;
+
 // Several sources: v[j][p] = m1 u1(j, p) + m2 u2(j, p), source-contiguous, so that a
 // row's entry reads the values of all its sources side by side (32 edges x 32 sources a
 // CTA, turned through shared memory).
@@ -180,52 +189,64 @@ __global__ void __launch_bounds__(256) k_history_combine(const double* __restric
   }
 }
 
-// rhs = C v + coef S for 32 rows a CTA, G lanes a row, a source per lane (32 sources at a
+// rhs = C v + coef S for R rows a CTA, G lanes a row, a source per lane (G sources at a
 // time): every entry is one contiguous read of its sources' values and there is nothing
-// to reduce; the results go through shared memory to the column-major right-hand side.
+// to reduce but, where R rows leave lanes, the SPLIT groups of G that share a row's entries;
+// the results go through shared memory to the column-major right-hand side.
 // Bound by the reads of v through L1 and L2 (33 entries x 8 npls bytes a row).  With a
 // warp a row over column-major vectors, every one of 32 lanes gathering its own entry for
 // eight sources in turn, this was 1,885 us at 345,744 edges and 32 sources; now 287 and
-// 54 for the combination above.
-template <int G>
+// 54 for the combination above (1,536,000 rows: 2 sources 1,689 and 296 us together, 505
+// without the split; 4 sources 2,039 and 375, 476).
+// DIRECT: v is formed on the way from the two layers, with fewer rows a CTA.
+template <int G, int R, bool DIRECT>
 __global__ void __launch_bounds__(256) k_history_rhs_multi(const int64_t* __restrict__ rowptr,
                                                            const int* __restrict__ col, const double* __restrict__ C,
-                                                           const double* __restrict__ v,
+                                                           const double* __restrict__ v, const double* __restrict__ u1,
+                                                           const double* __restrict__ u2, double m1c, double m2c,
                                                            const double* __restrict__ S, double coef,
                                                            const uint8_t* __restrict__ bound, int n, int npls,
                                                            double* __restrict__ rhs) {
-  __shared__ double out[32][33];  // [source][row]
-  const int row0 = blockIdx.x * 32, sub = threadIdx.x % G, grp = threadIdx.x / G;
-  for (int p0 = 0; p0 < npls; p0 += 32) {
+  constexpr int SPLIT = 256 / (G * R) > 1 ? 256 / (G * R) : 1, GROUPS = 256 / (G * SPLIT);
+  __shared__ double out[SPLIT][G][R + 1];  // [part][source][row]
+  const int row0 = blockIdx.x * R, sub = threadIdx.x % G, part = (threadIdx.x / G) % SPLIT;
+  for (int p0 = 0; p0 < npls; p0 += G) {
     const int p = p0 + sub;
-    for (int r = grp; r < 32; r += 256 / G) {
+    auto value = [&](int64_t j) {
+      if (!DIRECT) return __ldg(v + j * npls + p);
+      const int64_t off = j + (int64_t)p * n;
+      return m2c != 0.0 ? __ldg(u1 + off) * m1c + __ldg(u2 + off) * m2c : __ldg(u1 + off) * m1c;
+    };
+    for (int r = threadIdx.x / (G * SPLIT); r < R; r += GROUPS) {
       const int row = row0 + r;
       double acc[2] = {0.0, 0.0};
       if (row < n && !bound[row] && p < npls) {
-        const int64_t b = rowptr[row], e = rowptr[row + 1];
-        int64_t q = b;
-        for (; q + 4 <= e; q += 4) {
+        const int64_t e = rowptr[row + 1];
+        int64_t q = rowptr[row] + part;
+        for (; q + 3 * SPLIT < e; q += 4 * SPLIT) {
           int j[4];
           double c[4], x[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) j[i] = __ldg(col + q + i);
+          for (int i = 0; i < 4; ++i) j[i] = __ldg(col + q + i * SPLIT);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            c[i] = __ldg(C + q + i);
-            x[i] = __ldg(v + (int64_t)j[i] * npls + p);
+            c[i] = __ldg(C + q + i * SPLIT);
+            x[i] = value(j[i]);
           }
 #pragma unroll
           for (int i = 0; i < 4; ++i) acc[i & 1] = fma(c[i], x[i], acc[i & 1]);
         }
-        for (; q < e; ++q) acc[0] = fma(__ldg(C + q), __ldg(v + (int64_t)__ldg(col + q) * npls + p), acc[0]);
+        for (; q < e; q += SPLIT) acc[0] = fma(__ldg(C + q), value(__ldg(col + q)), acc[0]);
       }
-      out[sub][r] = acc[0] + acc[1];
+      out[part][sub][r] = acc[0] + acc[1];
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < 32 * min(G, npls - p0); q += 256) {
-      const int r = q & 31, pp = q >> 5, row = row0 + r;
+    for (int q = threadIdx.x; q < R * min(G, npls - p0); q += 256) {
+      const int r = q % R, pp = q / R, row = row0 + r;
       if (row < n) {
-        double t = out[pp][r];
+        double t = out[0][pp][r];
+#pragma unroll
+        for (int i = 1; i < SPLIT; ++i) t += out[i][pp][r];
         if (coef != 0.0 && !bound[row]) t += coef * S[row + (int64_t)(p0 + pp) * n];
         rhs[row + (int64_t)(p0 + pp) * n] = t;
       }
@@ -467,21 +488,29 @@ void launch_history_rhs(const int64_t* rowptr, const int* col, const double* Cva
                         cudaStream_t s) {
   if (npls > 1) {
     if (n <= 0) return;
-    const unsigned tiles = (unsigned)((n + 31) / 32);
-    k_history_combine<<<dim3(tiles, (unsigned)((npls + 31) / 32)), 256, 0, s>>>(u1, u2, m1c, m2c, n, npls, scratch);
-    auto go = [&](auto kernel) {
-      kernel<<<tiles, 256, 0, s>>>(rowptr, col, Cval, scratch, S, coef, bound, n, npls, rhs);
+    const bool direct = (int64_t)n * npls <= kDirectValues;
+    if (!direct)
+      k_history_combine<<<dim3((unsigned)((n + 31) / 32), (unsigned)((npls + 31) / 32)), 256, 0, s>>>(
+          u1, u2, m1c, m2c, n, npls, scratch);
+    auto go = [&](auto lanes) {
+      constexpr int G = decltype(lanes)::value, R = G <= 8 ? 8 : 64 / G;
+      if (direct)
+        k_history_rhs_multi<G, R, true><<<(unsigned)((n + R - 1) / R), 256, 0, s>>>(
+            rowptr, col, Cval, nullptr, u1, u2, m1c, m2c, S, coef, bound, n, npls, rhs);
+      else
+        k_history_rhs_multi<G, 32, false><<<(unsigned)((n + 31) / 32), 256, 0, s>>>(
+            rowptr, col, Cval, scratch, nullptr, nullptr, m1c, m2c, S, coef, bound, n, npls, rhs);
     };
     if (npls <= 2)
-      go(k_history_rhs_multi<2>);
+      go(std::integral_constant<int, 2>());
     else if (npls <= 4)
-      go(k_history_rhs_multi<4>);
+      go(std::integral_constant<int, 4>());
     else if (npls <= 8)
-      go(k_history_rhs_multi<8>);
+      go(std::integral_constant<int, 8>());
     else if (npls <= 16)
-      go(k_history_rhs_multi<16>);
+      go(std::integral_constant<int, 16>());
     else
-      go(k_history_rhs_multi<32>);
+      go(std::integral_constant<int, 32>());
   } else {
     const int64_t threads = (int64_t)n * kRhsLanes;
     k_history_rhs<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(rowptr, col, Cval, u1, u2, m1c, m2c, S, coef,

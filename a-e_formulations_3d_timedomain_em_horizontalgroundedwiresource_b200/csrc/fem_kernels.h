@@ -31,7 +31,7 @@ void launch_combine(const double* Cval, const double* Bval, const int64_t* src, 
 // History right-hand side for npls columns (column-major, leading dimension n):
 //   rhs = C * (m1 * u1 + m2 * u2) + coef * S, zero on Dirichlet rows
 // (CalcNonstat3DLine/time_approx.cpp:1018-1081).  With several columns scratch (n x npls
-// doubles, not u1, u2, S or rhs) holds m1 * u1 + m2 * u2 on the way.
+// doubles, not u1, u2, S or rhs) may hold m1 * u1 + m2 * u2 on the way.
 void launch_history_rhs(const int64_t* rowptr, const int* col, const double* Cval, const double* u1,
                         const double* u2, double m1, double m2, const double* S, double coef,
                         const uint8_t* bound, int n, int npls, double* rhs, double* scratch, cudaStream_t s);

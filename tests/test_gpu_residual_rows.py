@@ -41,12 +41,15 @@ def test_long_rows_against_extended_precision(pkg, kind, n, per_row, ncols):
     pkg.residual_norms(0, n, *[v.data_ptr() for v in dev], ld, ncols, norms.data_ptr(),
                        torch.cuda.current_stream().cuda_stream)
     got = norms.cpu().numpy()
-    first = np.minimum(ptr[:-1], max(ptr[-1] - 1, 0))
     u = 2.0 ** -53
+
+    def row_sums(p):  # (a zero behind the last entry, where empty rows at the end begin)
+        return np.where(lens > 0, np.add.reduceat(np.append(p, 0), ptr[:-1]), 0)
+
     for j in range(ncols):
         p = val * x[j, col].astype(np.longdouble)
-        r = b[j, :n] - np.where(lens > 0, np.add.reduceat(p, first), 0)
-        size = np.abs(b[j, :n]) + np.where(lens > 0, np.add.reduceat(np.abs(p), first), 0)
+        r = b[j, :n] - row_sums(p)
+        size = np.abs(b[j, :n]) + row_sums(np.abs(p))
         want = np.sqrt(np.sum(r * r))
         # a row's sum of L products errs by (L + 2) u of their sizes, and a sum of n squares,
         # which runs over at most 300 partial sums in a row, by 300 u of itself
