@@ -3219,6 +3219,15 @@ static size_t mail_bytes(const Symbolic& sy, int nrhs_max, int elem) {
   return (size_t)elem * 2 * (size_t)sy.n_flags * SB * std::min(nrhs_max, 2);
 }
 
+// The child-to-parent maps that set-up turns (setup_kids), and whether they find room in
+// the first slot's factor, which nothing uses before the first factorization.
+static size_t kid_map_bytes(const Symbolic& sy) {
+  return 8 * sy.rel_off.size() + 4 * (sy.front_parent.size() + sy.rel.size());
+}
+static bool kid_maps_in_factor(const Symbolic& sy, int elem) {
+  return kid_map_bytes(sy) <= (size_t)elem * (size_t)std::max<int64_t>(1, sy.nnz_l);
+}
+
 int64_t GpuCholesky::bytes_needed(const Symbolic& sy, int nrhs_max, int precision_bytes, int nslots,
                                   int factor_bytes) {
   const int64_t el = (precision_bytes == 4) ? 4 : 8, nr = std::max(1, nrhs_max);
@@ -3229,10 +3238,11 @@ int64_t GpuCholesky::bytes_needed(const Symbolic& sy, int nrhs_max, int precisio
   if (fel == 8) b += sy.oz_rows_max * ((int64_t)kOzModuli * kOzK + 4);  // residues + exponents
   b += 8 * (int64_t)sy.task_aux.size() + (int64_t)mail_bytes(sy, (int)nr, (int)el);
   b += 4 * sy.kid_rows + 8 * (int64_t)sy.front_m.size();  // child maps
+  if (!kid_maps_in_factor(sy, (int)el)) b += (int64_t)kid_map_bytes(sy);
   b += 8 * (int64_t)(sy.l_off.size() + sy.u_off.size() + sy.wvec_off.size() + sy.entry_dst.size() +
-                     sy.rel_off.size() + sy.rows_off.size() + sy.task_prefix.size() + sy.dinv_off.size());
-  b += 4 * (int64_t)(sy.front_m.size() + sy.front_k.size() + sy.rel.size() + sy.rows_all.size() + sy.tasks.size() +
-                     sy.front_parent.size() + sy.front_c0.size() + sy.solve_items.size() + sy.solve_units.size() +
+                     sy.rows_off.size() + sy.task_prefix.size() + sy.dinv_off.size());
+  b += 4 * (int64_t)(sy.front_m.size() + sy.front_k.size() + sy.rows_all.size() + sy.tasks.size() +
+                     sy.front_c0.size() + sy.solve_items.size() + sy.solve_units.size() +
                      max_col_groups((int)nr) * sync_ints(sy) + 4);
   return b;
 }
@@ -3320,15 +3330,21 @@ std::string GpuCholesky::setup_kids(cudaStream_t s) {
     ptr[f + 1] = (int)list.size();
   }
   std::string e;
-  int *parent = nullptr, *rel = nullptr;
-  int64_t* rel_off = nullptr;
   if (!(e = upload(&d_kid_ptr_, ptr, s)).empty()) return e;
   if (!(e = upload(&d_kid_list_, list, s)).empty()) return e;
   if (!(e = upload(&d_inv_off_, inv_off, s)).empty()) return e;
   if (!(e = alloc((void**)&d_inv_, sizeof(int) * (size_t)std::max<int64_t>(1, total))).empty()) return e;
-  if (!(e = upload(&parent, sy_.front_parent, s)).empty()) return e;
-  if (!(e = upload(&rel_off, sy_.rel_off, s)).empty()) return e;
-  if (!(e = upload(&rel, sy_.rel, s)).empty()) return e;
+  void* maps = d_L_[0];
+  if (!kid_maps_in_factor(sy_, elem_) && !(e = alloc(&maps, kid_map_bytes(sy_))).empty()) return e;
+  int64_t* rel_off = static_cast<int64_t*>(maps);
+  int* parent = reinterpret_cast<int*>(rel_off + sy_.rel_off.size());
+  int* rel = parent + sy_.front_parent.size();
+  auto put = [&](void* dst, const void* src, size_t bytes) {
+    return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s) : cudaSuccess;
+  };
+  TDEM_CUDA_TRY(put(rel_off, sy_.rel_off.data(), 8 * sy_.rel_off.size()));
+  TDEM_CUDA_TRY(put(parent, sy_.front_parent.data(), 4 * sy_.front_parent.size()));
+  TDEM_CUDA_TRY(put(rel, sy_.rel.data(), 4 * sy_.rel.size()));
   TDEM_CUDA_TRY(cudaMemsetAsync(d_inv_, 0xFF, sizeof(int) * (size_t)std::max<int64_t>(1, total), s));
   if (nf > 0) k_invert_rows<<<(unsigned)nf, 256, 0, s>>>(parent, rel_off, rel, d_inv_off_, d_inv_);
   TDEM_CUDA_TRY(cudaGetLastError());
