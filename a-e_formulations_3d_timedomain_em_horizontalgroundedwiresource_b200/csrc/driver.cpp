@@ -520,13 +520,13 @@ std::string TransientSolve::setup_device(cudaStream_t stream) {
   if (const char* ps = std::getenv("TDEM_PANEL_SOLVE")) chol_->set_panel_solve(ps[0] == '1');
   if (const char* la = std::getenv("TDEM_LOOKAHEAD")) chol_->set_lookahead(la[0] != '0');
   if (const char* at = std::getenv("TDEM_SOLVE_AUTOTUNE")) chol_->set_autotune(at[0] != '0');
-  if (const char* fs = std::getenv("TDEM_SOLVE_SCHEDULE")) {  // "kind,split": a fixed schedule
+  if (const char* fs = std::getenv("TDEM_SOLVE_SCHEDULE")) {  // "kind,split[,groups]": a fixed schedule
     SolveSchedule sc;
-    if (std::sscanf(fs, "%d,%d", &sc.kind, &sc.split) == 2 && sc.kind >= 0 && sc.kind <= 2 && sc.split >= 1 &&
-        sc.split <= kMaxRhs)
+    if (std::sscanf(fs, "%d,%d,%d", &sc.kind, &sc.split, &sc.groups) >= 2 && sc.kind >= 0 && sc.kind <= 2 &&
+        sc.split >= 1 && sc.split <= kMaxRhs && (sc.groups == 0 || sc.groups == 1 || sc.groups == 2 || sc.groups == 4))
       chol_->force_schedule(sc);
     else
-      return "TDEM_SOLVE_SCHEDULE must be \"kind,split\" with kind 0, 1 or 2";
+      return "TDEM_SOLVE_SCHEDULE must be \"kind,split[,groups]\" with kind 0, 1 or 2 and groups 0, 1, 2 or 4";
   }
   // with a factorization on the FP64 tensor pipe running beside the steps, the level
   // solves keep one CTA per SM so its kernels can share every SM (with the

@@ -2980,23 +2980,6 @@ inline int64_t sync_ints(const Symbolic& sy) {
 }
 // Column groups of the many-column solves: groups of at least 8 columns, at most four.
 inline int max_col_groups(int nrhs) { return nrhs > 16 ? 4 : (nrhs > 8 ? 2 : 1); }
-// A level's groups run side by side, each with a chain of its own over fewer columns: a
-// link is about 3.2 us and 0.17 us a column.  Each group reads the level's factor, about
-// 4 TB/s: the fewest groups that leave the slower of the two least.
-inline int col_groups(const LevelPlan& lp, int nrhs) {
-  int best = 1;
-  double least = 0;
-  for (int g = 1; g <= max_col_groups(nrhs); g *= 2) {
-    const double cols = (nrhs + g - 1) / g;
-    const double us = std::max((double)lp.chain * (3.2 + 0.17 * cols), g * 8.0 * (double)lp.entries / 4e6);
-    if (g == 1 || us < 0.95 * least) {
-      least = us;
-      best = g;
-    }
-  }
-  return best;
-}
-
 // One forward and one backward launch per level (plus the front-vector set-up).
 // STREAM: the persistent streaming kernels (nrhs <= NR <= 4, grid = resident
 // CTAs); MR: the persistent many-column kernels (FP64, 3..32 columns, grid =
@@ -3006,7 +2989,7 @@ template <class T, int RPT, bool STREAM, bool MR = false>
 void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T* part, const double* b, double* x,
                          SolveArgs a, const Kids& kids, const int* tasks,
                          const int64_t* prefix, FusedArgs fa, int* sync, const int (&resident)[2], Launched& done,
-                         cudaStream_t s) {
+                         cudaStream_t s, [[maybe_unused]] int col_groups = 0) {
   static_assert(!MR || std::is_same<T, double>::value, "the many-column persistent kernels are FP64");
   const int nlev = (int)sy.levels.size();
   int* tickets = sync;
@@ -3021,6 +3004,9 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
   auto grid = [&](int64_t count, int dir) {
     return (STREAM || MR) ? (unsigned)std::min<int64_t>(count, resident[dir]) : grid_of(count);
   };
+  [[maybe_unused]] auto groups_of = [&](const LevelPlan& lp) {
+    return col_groups > 0 ? std::min(col_groups, max_col_groups(a.nrhs)) : solve_column_groups(lp, a.nrhs);
+  };
   for (int l = 0; l < nlev; ++l) {
     const LevelPlan& lp = sy.levels[l];
     if (lp.assemble.ctas == 0) continue;  // only fronts without rows
@@ -3033,7 +3019,7 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
     f.ticket = tickets + 2 * l;
     f.flags = fflags;
     if constexpr (MR) {
-      const int groups = col_groups(lp, a.nrhs);
+      const int groups = groups_of(lp);
       f.cols = (a.nrhs + groups - 1) / groups;
       auto go = [&](auto kernel) {
         done.add(launch_next(kernel, dim3((unsigned)std::min<int64_t>(lp.fwd_count, std::max(1,
@@ -3060,7 +3046,7 @@ void launch_level_solves(const Symbolic& sy, const T* L, const T* Dinv, T* W, T*
     f.flags = bflags;
     f.mail = static_cast<char*>(fa.mail) + mail;
     if constexpr (MR) {
-      const int groups = col_groups(lp, a.nrhs);
+      const int groups = groups_of(lp);
       f.cols = (a.nrhs + groups - 1) / groups;
       auto go = [&](auto kernel) {
         done.add(launch_next(kernel, dim3((unsigned)std::min<int64_t>(lp.bwd_count, std::max(1,
@@ -3108,10 +3094,10 @@ Launched launch_solve_fused(const Symbolic& sy, const T* L, const T* Dinv, T* W,
 // The persistent many-column level solves (FP64, 3 <= nrhs <= 32).
 Launched launch_solve_mr(const Symbolic& sy, const double* L, const double* Dinv, double* W, double* part, const double* b,
                     double* x, SolveArgs a, const Kids& kids, const int* tasks, const int64_t* prefix, FusedArgs fa, int* sync, const int (&resident)[2],
-                    cudaStream_t s) {
+                    cudaStream_t s, int col_groups) {
   Launched done;
   launch_level_solves<double, 8, false, true>(sy, L, Dinv, W, part, b, x, a, kids, tasks, prefix, fa, sync, resident,
-                                              done, s);
+                                              done, s, col_groups);
   return done;
 }
 
@@ -3179,6 +3165,23 @@ std::string set_fused_attributes() {
 }
 
 }  // namespace
+
+// A level's groups run side by side, each with a chain of its own over fewer columns: a
+// link is about 3.2 us and 0.17 us a column.  Each group reads the level's factor, about
+// 4 TB/s: the fewest groups that leave the slower of the two least.
+int solve_column_groups(const LevelPlan& lp, int nrhs) {
+  int best = 1;
+  double least = 0;
+  for (int g = 1; g <= max_col_groups(nrhs); g *= 2) {
+    const double cols = (nrhs + g - 1) / g;
+    const double us = std::max((double)lp.chain * (3.2 + 0.17 * cols), g * 8.0 * (double)lp.entries / 4e6);
+    if (g == 1 || us < 0.95 * least) {
+      least = us;
+      best = g;
+    }
+  }
+  return best;
+}
 
 GpuCholesky::~GpuCholesky() {
   for (SolveGraph& g : graph_)
@@ -3464,7 +3467,7 @@ cudaError_t GpuCholesky::solve_with(const SolveSchedule& sc, const double* d_b, 
     for (int d = 0; d < 2; ++d)
       res[d] = solve_ctas_cap_ > 0 ? std::min(resident_mr_[d], solve_ctas_cap_ * sms_) : resident_mr_[d];
     done = launch_solve_mr(sy_, (const double*)Lp, (const double*)Dp, (double*)d_W_, (double*)d_spart_,
-                           d_b, d_x, a, kids, d_tasks_, d_prefix_, fa, d_sync_, res, s);
+                           d_b, d_x, a, kids, d_tasks_, d_prefix_, fa, d_sync_, res, s, sc.groups);
   } else if (sc.kind != 1) {
     FusedArgs fa{d_units_, 0, nullptr, nullptr, nullptr, d_err_ + 1};
     fa.mail = d_mail_;

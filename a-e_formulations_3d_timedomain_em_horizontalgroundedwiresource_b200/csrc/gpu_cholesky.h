@@ -29,8 +29,14 @@ struct SolveSchedule {
                   //    columns per group: CTAs stay resident and stream their units'
                   //    blocks through shared-memory stages)
   int split = 1;  // the columns are solved in this many groups one after another
+  int groups = 0;  // kind 2: column groups side by side on every level (0: solve_column_groups;
+                   // never more than that may give)
   float ms = 0;   // measured device time of one solve with this schedule (0: not measured)
 };
+
+// Column groups side by side (1, 2 or 4) that a level of the persistent many-column solves
+// takes for nrhs columns.
+int solve_column_groups(const LevelPlan& lp, int nrhs);
 
 class GpuCholesky {
  public:
