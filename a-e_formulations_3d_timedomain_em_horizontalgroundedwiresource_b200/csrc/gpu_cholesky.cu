@@ -2299,7 +2299,9 @@ __global__ void __launch_bounds__(256, 2) k_bwd_stream(const T* __restrict__ L, 
 // Diagonal inverses of final pivot units are held in registers from the start and
 // applied on the FP64 tensor pipe like the blocks (as 64 multiply-adds per value on the
 // CUDA cores, each with its own shared-memory operand, they were half of a chain link).
-// Products and sums are those of k_fwd_level / k_bwd_level but for the inverses' order.
+// Products and sums are those of k_fwd_level / k_bwd_level, which apply the inverses by
+// chains of multiply-adds: the tensor pipe's own order inside an instruction is not
+// documented, and has given the same bits wherever the two were compared.
 // ---------------------------------------------------------------------------
 constexpr int kMrStages = 2;
 constexpr int kMrYld = ys_ld(32);  // solution-block stage leading dimension (32 columns)
@@ -2401,8 +2403,8 @@ __global__ void __launch_bounds__(256, 2) k_fwd_mrhs(const double* __restrict__ 
 #pragma unroll
     for (int j = 0; j < RPT; ++j) tot[j] = 0.0;
     if (fin) gather_partials<double, RPT>(my_part, u.nparts, nr_rhs, fa.counters + u.cnt, fa.err, tot, nr_all);
-    // flags of a front are set in chain order: the newest flag of the range stands
-    // for all of them (see k_fwd_stream)
+    // the flags of a front are set in chain order (the unit that sets flag q has waited for
+    // flag q - 1), so the newest flag of the range stands for all of them
     const bool chain = fin && piv;
     if (t == 0) {
       int ready = 1;
@@ -2582,8 +2584,8 @@ __global__ void __launch_bounds__(256, 2) k_bwd_mrhs(const double* __restrict__ 
 #pragma unroll
     for (int j = 0; j < RPT; ++j) tot[j] = 0.0;
     if (fin) gather_partials<double, RPT>(my_part, u.nparts, nr_rhs, fa.counters + u.cnt, fa.err, tot, nr_all);
-    // flags are set last column first: flag lo stands for every pivot row block of
-    // the range (see k_bwd_stream); update rows need no flag
+    // flags are set last column first (the unit that sets flag q has waited for flag q + 1):
+    // flag lo stands for every pivot row block of the range; update rows need no flag
     if (t == 0) {
       int ready = 1;
       if (lo < hi && lo < pb) {

@@ -11,11 +11,12 @@
 // Chinese remainder theorem gives
 //   Q_a . Q_b / P = sum_l acc_l T_l  (mod 1),   T_l = ((P / p_l)^-1 mod p_l) / p_l,
 // which the epilogue sums in 64-bit fixed point (and a float below it) straight from the int32 accumulators
-// (no reduction modulo p_l: an accumulator only matters modulo p_l).  The T_l are
-// kept to 2^-88, and the sum is within 2^-62 P of the product at worst and 2^-67 P for
-// accumulators of usual size: below the rounding of the rows to integers, an error of at most 2^-62 |row| per
-// entry where a double's own is 2^-53 |entry|.  What remains is one FP64 rounding of the product and
-// one of the subtraction.
+// (no reduction modulo p_l: an accumulator only matters modulo p_l).  The sum errs by at
+// most 2^-60.8 P (the float's roundings with all 16 accumulators at their largest 8.6 units
+// of 2^-64, the T_l, kept to 2^-88, 0.4) and by 2^-68 P for accumulators of usual size.  The
+// rounding of a row to integers errs by at most 2^-62 of the row's norm per entry, 2^-57.6 of
+// it over 512 entries, where a row of doubles is known to 2^-53.  What remains is one FP64
+// rounding of the product and one of the subtraction.
 //
 // Against digit splitting (eight 7-bit digits, 36 products of one output tile), which
 // this replaces, the tensor pipe does 16 products instead of 36, and because the

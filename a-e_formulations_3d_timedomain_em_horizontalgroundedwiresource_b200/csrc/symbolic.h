@@ -34,6 +34,11 @@ constexpr int kSolveLookahead = 8;  // extra blocks a chain unit takes ahead of 
 // of the outer panel is scaled by a power of two, rounded to integers and reduced
 // modulo kOzModuli moduli; the steps of at least kOzMinFlops flops take that path, in
 // launches whose panels total at most kOzRowsCap rows (the residue buffer: 1.07 GB).
+// Steps that take the path are rounded once an entry, the others (FP64 tensor pipe) once a
+// product, so the line lies as low as it costs little.  (Runs in ms at 0.5e9 / 1e9 / 2e9 /
+// 4e9 / 8e9 flops / no step: 40^3 cells 204 / 204 / 199 / 196 / 195 / 240, 48^3 and 32 wires
+// 212 / 213 / 210 / 209 / 205 / 256, 35^3 at precision 32 56.1 / 54.5 / 53.7 / 53.6 / 53.8 /
+// 63.8, 80^3 837 / 837 / 839 / 837 / 836 / 1,539.)
 constexpr int kOzModuli = 16;
 constexpr int kOzK = kOuter;          // residues per row and modulus (K of an outer panel, padded)
 constexpr int64_t kOzRowsCap = 1 << 17;
